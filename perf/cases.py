@@ -167,6 +167,7 @@ def prepare(case, seed):
             seen = (slice(None),) * (1 if path == "decode" else 2) + (slice(0, case["pos"]),)
             for cache in (model.k_cache, model.v_cache):
                 cache[seen] = torch.randn(cache[seen].shape, dtype=torch.float16, device="cuda", generator=gen)
+            torch.cuda.synchronize()   # capture() takes its warm-up step on a stream of its own
             model.capture()
             state = {"model": model, "pos": torch.full_like(model.pos, case["pos"]),
                      "token": torch.randint(0, case["vocab"], model.token.shape, device="cuda", generator=gen)}
@@ -242,3 +243,84 @@ def tolerance(case):
         small_batch = case["rows"] > 1 and case.get("layout", "row") == "row"
         return {"rel": 1.7e-3, "max": 9e-3} if small_batch else {"rel": 8.5e-4, "max": 2e-3}
     return {"decode": {"rel": 1.4e-2, "max": 6.5e-2}, "batch": {"rel": 1.8e-2, "max": 9e-2}, "prefill": {"rel": 7e-3, "max": 4e-2}}[path]
+
+
+# ---- the same in 64 bits, in plain torch ------------------------------------------------------------------------------
+def _dense(packed, scales):
+    """Packed planes [K/32, q, N] and scales [., q, .] (rows of the scales: equal runs of K, columns: equal runs of N) as a float64 weight [K, N]."""
+    words, q, n = packed.shape
+    k = 32 * words
+    shifts = torch.arange(32, device=packed.device, dtype=torch.int32).view(1, 32, 1)
+    weight = torch.zeros(k, n, dtype=torch.float64, device=packed.device)
+    for b in range(q):
+        a = scales[:, b].double().repeat_interleave(n // scales.shape[2], dim=1)   # [runs of K, N]
+        for lo in range(0, words, 128):
+            sign = ((packed[lo:lo + 128, b][:, None, :] >> shifts) & 1).reshape(-1, n).double().mul_(2).sub_(1)
+            rows = torch.arange(32 * lo, 32 * lo + sign.shape[0], device=packed.device) // (k // scales.shape[0])
+            weight[32 * lo:32 * lo + sign.shape[0]] += sign.mul_(a[rows])
+    return weight
+
+
+def _layer(lin, x):
+    a = lin.alpha
+    if a.dtype == torch.int8:   # three exponents a multiplier, -128 for one that is not there
+        a = torch.where(a == -128, torch.zeros((), dtype=torch.float64, device=a.device), torch.exp2(a.double())).sum(-1)
+    y = x @ _dense(lin.binaryWeight, a)
+    return y if lin.bias is None else y + lin.bias.double()
+
+
+def _norm(x, w, eps):
+    return x * torch.rsqrt((x * x).mean(-1, keepdim=True) + eps) * w.double()
+
+
+def _tokens(model, shape, ids, keys, values, first):
+    """`ids` [sequences, tokens] at positions first, first + 1, ..: the logits of the last token of each sequence; their keys
+    and values are written into `keys`, `values` [layers, sequences, positions, kv heads, head dim]."""
+    hd, kvh, rep = shape.head_dim, shape.kv_heads, shape.heads // shape.kv_heads
+    s, t = ids.shape
+    dev = ids.device
+    at = torch.arange(first, first + t, device=dev)
+    angle = at.double()[:, None] / shape.rope_theta ** (torch.arange(0, hd, 2, device=dev).double() / hd)
+    cos, sin = angle.cos()[None, :, None], angle.sin()[None, :, None]
+
+    def turned(v, heads):
+        a, b = v.view(s, t, heads, 2, hd // 2).unbind(3)
+        return torch.cat((a * cos - b * sin, b * cos + a * sin), dim=-1)
+
+    later = torch.arange(first + t, device=dev)[None, :] > at[:, None]
+    x = model.embed[ids].double()
+    for i, blk in enumerate(model.blocks):
+        h = _norm(x, blk.input_norm, shape.eps)
+        qh = turned(_layer(blk.q_proj, h), shape.heads)
+        keys[i, :, first:first + t] = turned(_layer(blk.k_proj, h), kvh)
+        values[i, :, first:first + t] = _layer(blk.v_proj, h).view(s, t, kvh, hd)
+        k, v = (c[i, :, :first + t].double().repeat_interleave(rep, dim=2) for c in (keys, values))
+        scores = torch.einsum("sthd,sphd->shtp", qh, k) / math.sqrt(hd)
+        p = torch.softmax(scores.masked_fill(later, float("-inf")), dim=-1)
+        x = x + _layer(blk.o_proj, torch.einsum("shtp,sphd->sthd", p, v).reshape(s, t, -1))
+        h = _norm(x, blk.post_norm, shape.eps)
+        x = x + _layer(blk.down_proj, torch.nn.functional.silu(_layer(blk.gate_proj, h)) * _layer(blk.up_proj, h))
+    return _norm(x[:, -1], model.final_norm, shape.eps) @ model.lm_head.double().t()
+
+
+def exact(case, seed):
+    path, state = case["path"], prepare(case, seed)
+    with torch.no_grad():
+        if path == "linear":
+            return _layer(state["layer"], state["x"].double())
+        if path == "set":
+            out = []
+            for launch in state["sequence"]._launches:
+                for _, bits, scales, _, x, _ in launch._keep:
+                    out.append(x.double() @ _dense(bits, scales))
+            return out
+        if path == "convert":
+            return None, state["alpha"].double().transpose(1, 2)
+        model, shape = state["model"], _shape(case)
+        keys, values = model.k_cache.float(), model.v_cache.float()   # given ones are fp16 numbers; those computed here are rounded to 32 bits
+        if path == "batch":
+            logits = _tokens(model, shape, state["token"].view(-1, 1), keys, values, case["pos"])
+        else:
+            ids, first = (state["ids"], 0) if path == "prefill" else (state["token"], case["pos"])
+            logits = _tokens(model, shape, ids.view(1, -1), keys[:, None], values[:, None], first)[0]
+        return {"logits": logits, "keys": keys, "values": values}
