@@ -37,6 +37,10 @@ int sal_pack_planes_i8(const void *signs, void *out, int R, int C, int q, int ke
  */
 int sal_repack_lat_to_kernel(const void *in, void *out, int K, int N, int q, void *stream);
 
+/* sal_repack_lat_to_kernel and, in the same launch, the scales fp32 [R][G][q] -> fp32 [R][q][G] (what
+ * lut_gemm/kernel.py:112-133 does with both tensors of a checkpoint). */
+int sal_convert_lat(const void *in, void *out, const void *alpha, void *alpha_out, int K, int N, int q, int R, int G, void *stream);
+
 #ifdef __cplusplus
 }
 #endif

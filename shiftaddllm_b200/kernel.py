@@ -138,6 +138,15 @@ def convert_weight(BinaryWeight: torch.Tensor, Alpha: torch.Tensor):
 
         src = BinaryWeight.contiguous()
         out = torch.empty((k_in // 32, q, w * 32), dtype=torch.int32, device=src.device)
+        # scales as the checkpoints hold them ride in the same launch
+        if Alpha.device == src.device and Alpha.dtype == torch.float32 and Alpha.dim() == 3 and Alpha.shape[2] == q and Alpha.numel() > 0 \
+                and Alpha.is_contiguous() and not Alpha.requires_grad:
+            alpha_out = torch.empty((Alpha.shape[0], q, Alpha.shape[1]), dtype=torch.float32, device=src.device)
+            with torch.cuda.device(src.device):
+                _lib.check(_lib.load().sal_convert_lat(src.data_ptr(), out.data_ptr(), Alpha.data_ptr(), alpha_out.data_ptr(), k_in, w * 32, q,
+                                                       Alpha.shape[0], Alpha.shape[1],
+                                                       torch.cuda.current_stream(src.device).cuda_stream), "sal_convert_lat")
+            return out, alpha_out
         with torch.cuda.device(src.device):
             _lib.check(_lib.load().sal_repack_lat_to_kernel(src.data_ptr(), out.data_ptr(), k_in, w * 32, q,
                                                            torch.cuda.current_stream(src.device).cuda_stream),
