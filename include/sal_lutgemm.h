@@ -66,7 +66,11 @@ extern "C" {
 #define SAL_SWIGLU_FIXED 16u   /* with sal_problem.x_mul: x and x_mul are such INT64 accumulators (written with
                                   SAL_OUT_FIXED_ATOMIC), rounded to fp16 before silu(x) * x_mul is formed */
 
+#define SAL_MANY_ROWS 32u      /* sal_lutgemv_grouped / sal_prepare_grouped: M may exceed SAL_MAX_M, up to SAL_MAX_ROWS (plain
+                                  products; the tensor-core kernel's shapes, see sal_lutgemm_rows) */
+
 #define SAL_MAX_Q 8
+#define SAL_MAX_ROWS 4096
 #define SAL_MAX_M 64
 #define SAL_MAX_GROUP 8 /* problems per grouped launch */
 #define SAL_MAX_PEERS 8 /* GPUs taking part in a fused exchange */
@@ -167,6 +171,18 @@ int sal_lutgemm_block_shift(const void *bw, const void *alpha_u16, const void *b
 int sal_lutgemm_block_shift_int8(const void *bw, const void *alpha_i8, const void *bias, const void *x, void *y,
                                  int M, int K, int N, int q, int num_groups, int num_apot, unsigned flags,
                                  void *workspace, size_t workspace_bytes, void *stream);
+
+/*
+ * The tensor-core product by itself, for up to SAL_MAX_ROWS activation rows in one call (the entries above take
+ * SAL_MAX_M).  alpha_layout 0: fp16 [num_groups][q][N], groups along K of a multiple of 32 features; 1: fp16
+ * [K/8][q][num_groups], 2: uint16 (three 3-bit exponents) of that shape, groups along N of a multiple of 16 columns.
+ * x must be 16-byte aligned and q <= 4; what it does not take is SAL_E_UNSUPPORTED.  The result has the value of
+ * sal_lutgemv_shift_scale / sal_lutgemm_block / sal_lutgemm_block_shift on the same rows.  With less scratch than
+ * sal_lutgemm_rows_workspace_bytes(M) (zero-filled once, as above) fewer SMs share the work.
+ */
+size_t sal_lutgemm_rows_workspace_bytes(int M);
+int sal_lutgemm_rows(int alpha_layout, const void *bw, const void *alpha, const void *bias, const void *x, void *y, int M, int K, int N,
+                     int q, int num_groups, unsigned flags, void *workspace, size_t workspace_bytes, void *stream);
 
 /*
  * Grouped mode-A launch: up to SAL_MAX_GROUP independent products in ONE kernel

@@ -17,10 +17,11 @@ LIB_PATH = os.environ.get("SAL_LUTGEMM_LIBRARY") or os.path.join(_PKG_DIR, "libs
 SAL_OK = 0
 SAL_E_NULL, SAL_E_SHAPE, SAL_E_ALIGN, SAL_E_WORKSPACE = -1, -2, -3, -4
 SAL_E_LAUNCH, SAL_E_UNSUPPORTED, SAL_E_DEVICE, SAL_E_TIMEOUT = -5, -6, -7, -8
-SAL_ACCUMULATE, SAL_PDL, SAL_FORCE_GENERIC, SAL_OUT_FIXED_ATOMIC, SAL_SWIGLU_FIXED = 1, 2, 4, 8, 16
+SAL_ACCUMULATE, SAL_PDL, SAL_FORCE_GENERIC, SAL_OUT_FIXED_ATOMIC, SAL_SWIGLU_FIXED, SAL_MANY_ROWS = 1, 2, 4, 8, 16, 32
 SAL_MAX_GROUP = 8
 SAL_MAX_PEERS = 8
 SAL_MAX_M = 64
+SAL_MAX_ROWS = 4096   # rows of one tensor-core product (sal_lutgemm_rows)
 
 _vp, _i, _u, _sz = ctypes.c_void_p, ctypes.c_int, ctypes.c_uint, ctypes.c_size_t
 
@@ -54,6 +55,8 @@ SIGNATURES = {
     "sal_lutgemm_block": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _u, _vp, _sz, _vp]),
     "sal_lutgemm_block_shift": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _u, _vp, _sz, _vp]),
     "sal_lutgemm_block_shift_int8": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _u, _vp, _sz, _vp]),
+    "sal_lutgemm_rows_workspace_bytes": (_sz, [_i]),
+    "sal_lutgemm_rows": (_i, [_i, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _u, _vp, _sz, _vp]),
     "sal_lutgemv_grouped": (_i, [ctypes.POINTER(SalProblem), _i, _u, _vp, _sz, _vp]),
     "sal_lutgemv_grouped_exchange": (_i, [ctypes.POINTER(SalProblem), _i, _u, _vp, _sz, ctypes.POINTER(SalExchange),
                                           ctypes.POINTER(_i), _vp]),

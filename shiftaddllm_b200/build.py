@@ -12,8 +12,9 @@ import sys
 
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 REPO_DIR = os.path.dirname(PKG_DIR)
-SRCS = [os.path.join(PKG_DIR, "csrc", name) for name in ("sal_lutgemm.cu", "sal_decode_ops.cu", "sal_pack.cu")]
+SRCS = [os.path.join(PKG_DIR, "csrc", name) for name in ("sal_lutgemm.cu", "sal_mma.cu", "sal_decode_ops.cu", "sal_pack.cu")]
 HDRS = [os.path.join(REPO_DIR, "include", name) for name in ("sal_lutgemm.h", "sal_decode_ops.h", "sal_pack.h")]
+HDRS.append(os.path.join(PKG_DIR, "csrc", "sal_mma.h"))
 LIB = os.path.join(PKG_DIR, "libsal_lutgemm.so")
 
 NVCC_FLAGS = [
@@ -22,7 +23,7 @@ NVCC_FLAGS = [
     "-Xcompiler", "-fPIC", "-shared",
     "-Xlinker", "-soname=libsal_lutgemm.so",   # the compiled `lutgemm` module links to the library by this name
     "-cudart", "static",
-    "--threads", "0",   # the three translation units compile side by side
+    "--threads", "0",   # the translation units compile side by side
     "-U__CUDA_NO_HALF_OPERATORS__", "-U__CUDA_NO_HALF_CONVERSIONS__",
 ]
 

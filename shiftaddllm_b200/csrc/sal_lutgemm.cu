@@ -43,6 +43,7 @@
 #include <type_traits>
 
 #include "sal_lutgemm.h"
+#include "sal_mma.h"
 
 namespace {
 
@@ -1484,23 +1485,7 @@ typedef CUresult (*TensorMapEncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, c
 TensorMapEncodeTiledFn g_encode_tiled = nullptr;
 
 int encode_weight_map(CUtensorMap *out, const void *bw, int K, int N, int q) {
-    if (!g_encode_tiled) {
-        void *fn = nullptr;
-        cudaDriverEntryPointQueryResult qres;
-        if (!cuda_ok(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres)) ||
-            qres != cudaDriverEntryPointSuccess || fn == nullptr)
-            return SAL_E_LAUNCH;
-        g_encode_tiled = reinterpret_cast<TensorMapEncodeTiledFn>(fn);
-    }
-    // [K/32 words][q planes][N columns], innermost first; strides in bytes of all but the innermost dimension
-    const cuuint64_t dims[3] = {(cuuint64_t)N, (cuuint64_t)q, (cuuint64_t)(K / 32)};
-    const cuuint64_t strides[2] = {(cuuint64_t)N * 4, (cuuint64_t)N * 4 * (cuuint64_t)q};  // N % 4 == 0 keeps them multiples of 16
-    const cuuint32_t box[3] = {(cuuint32_t)BOX_COLS, (cuuint32_t)planes_per_slot(q), (cuuint32_t)KB_WORDS};
-    const cuuint32_t estr[3] = {1, 1, 1};
-    const CUresult r = g_encode_tiled(out, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, const_cast<void *>(bw), dims, strides, box,
-                                      estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS ? SAL_OK : SAL_E_LAUNCH;
+    return sal_encode_planes(out, bw, K, N, q, BOX_COLS, planes_per_slot(q), KB_WORDS);
 }
 
 template <int Q, int NCW, bool ABS, int ROWS, int SWIGLU, bool EXCH = false, bool ATOMIC = false, bool BLK = false>
@@ -1572,9 +1557,9 @@ bool tiled_eligible(const void *bw, const void *alpha, const void *bias, const v
     return true;
 }
 
-int validate_common(const void *bw, const void *alpha, const void *x, const void *y, int M, int K, int N, int q) {
+int validate_common(const void *bw, const void *alpha, const void *x, const void *y, int M, int K, int N, int q, int max_m = SAL_MAX_M) {
     if (!bw || !alpha || !x || !y) return SAL_E_NULL;
-    if (M < 1 || M > SAL_MAX_M || K <= 0 || N <= 0 || q < 1 || q > SAL_MAX_Q) return SAL_E_SHAPE;
+    if (M < 1 || M > max_m || K <= 0 || N <= 0 || q < 1 || q > SAL_MAX_Q) return SAL_E_SHAPE;
     if (K % 32 != 0) return SAL_E_SHAPE;
     if (!aligned(bw, 4) || !aligned(x, 2) || !aligned(y, 2)) return SAL_E_ALIGN;
     return SAL_OK;
@@ -1808,6 +1793,36 @@ int run_tiled_group(const sal_problem *problems, int count, unsigned flags, void
     return launch_built(L, workspace, ws_bytes, -1, stream);
 }
 
+// Products of several activation rows go to the tensor cores (sal_mma.cu) from this many rows on.  There the time hardly depends on the
+// rows, here it is a pass over all lookups per pair of rows (ROW; per row in the block layouts).  Times in us for 2 / 4 / 6 / 8 / 16 rows,
+// 4096 x 11008, 4 planes: tables 15 / 20 / 27 / 31 / 54, tensor cores 27 at all of them; 28672 x 8192, 2 planes: 32 / 45 / 58 / 74 / 132
+// against 70; block layout (16 columns), 4096 x 4096, 3 planes, 3 / 4 / 8 rows: 15 / 18 / 30 against 16.  Shapes that the tiled
+// table kernel does not take ran on the generic one, row by row: 2080 x 1378, 3 planes, 3 rows, 21 against 18.
+#ifdef SAL_MEASURE
+int g_mma_min_rows = 7, g_mma_min_rows_block = 4, g_mma_min_rows_generic = 2;
+#else
+constexpr int g_mma_min_rows = 7, g_mma_min_rows_block = 4, g_mma_min_rows_generic = 2;
+#endif
+bool mma_wanted(const sal_problem *problems, int count, unsigned flags, sal_mma::AlphaLayout layout, bool tiled) {
+    if (flags & (SAL_FORCE_GENERIC | SAL_OUT_FIXED_ATOMIC | SAL_SWIGLU_FIXED)) return false;
+    const int min_rows = !tiled ? g_mma_min_rows_generic : layout == sal_mma::ROW ? g_mma_min_rows : g_mma_min_rows_block;
+    for (int i = 0; i < count; ++i) {
+        const sal_problem &p = problems[i];
+        if (p.M < min_rows || !sal_mma::eligible(p.bw, p.alpha, p.x, p.M, p.K, p.N, p.q, p.num_groups, layout)) return false;
+    }
+    return true;
+}
+int run_mma_group(const sal_problem *problems, int count, sal_mma::AlphaLayout layout, unsigned flags, void *workspace, size_t ws_bytes,
+                  cudaStream_t stream) {
+    DeviceInfo *dev = nullptr;
+    int rc = device_info(&dev);
+    if (rc != SAL_OK) return rc;
+    sal_mma::Built b;
+    rc = sal_mma::build(problems, count, layout, flags, workspace ? ws_bytes : 0, dev->sms, &b);
+    if (rc != SAL_OK) return rc;
+    return sal_mma::launch(b, workspace, ws_bytes, stream);
+}
+
 // Problems of one grouped call sorted into classes of equal plane count q (each class is one kernel launch),
 // keeping the caller's order inside a class.  Returns the number of classes.
 int split_by_q(const sal_problem *problems, int count, sal_problem (*classes)[SAL_MAX_GROUP], int *sizes, int (*index)[SAL_MAX_GROUP]) {
@@ -1822,18 +1837,23 @@ int split_by_q(const sal_problem *problems, int count, sal_problem (*classes)[SA
     return nclass;
 }
 
-int validate_grouped(const sal_problem *problems, int count, bool exchange) {
+int validate_grouped(const sal_problem *problems, int count, unsigned flags, bool exchange) {
+    const bool many = (flags & SAL_MANY_ROWS) != 0;
     if (!problems) return SAL_E_NULL;
     if (count < 1 || count > SAL_MAX_GROUP) return SAL_E_SHAPE;
     for (int i = 0; i < count; ++i) {
         const sal_problem &sp = problems[i];
-        int rc = validate_common(sp.bw, sp.alpha, sp.x, sp.y, sp.M, sp.K, sp.N, sp.q);
+        int rc = validate_common(sp.bw, sp.alpha, sp.x, sp.y, sp.M, sp.K, sp.N, sp.q, many ? sal_mma::MAX_ROWS : SAL_MAX_M);
         if (rc != SAL_OK) return rc;
         if (sp.num_groups <= 0 || sp.K % sp.num_groups != 0) return SAL_E_SHAPE;
         if (sp.M != problems[0].M) return SAL_E_UNSUPPORTED;
         if (exchange && (sp.M != 1 || sp.x_mul != nullptr)) return SAL_E_UNSUPPORTED;
         if (sp.x_mul && !aligned(sp.x_mul, 16)) return SAL_E_ALIGN;
         if ((sp.x_mul != nullptr) != (problems[0].x_mul != nullptr)) return SAL_E_UNSUPPORTED;
+        if (sp.M > SAL_MAX_M) {   // only the tensor-core product takes so many rows
+            if (exchange || !mma_wanted(&sp, 1, flags, sal_mma::ROW, true)) return SAL_E_UNSUPPORTED;
+            continue;
+        }
         if (!tiled_eligible(sp.bw, sp.alpha, sp.bias, sp.x, sp.y, sp.M, sp.K, sp.N, sp.q, sp.num_groups))
             return SAL_E_UNSUPPORTED;
     }
@@ -1841,6 +1861,42 @@ int validate_grouped(const sal_problem *problems, int count, bool exchange) {
 }
 
 }  // namespace
+
+static int tensor_map_encoder() {
+    if (g_encode_tiled) return SAL_OK;
+    void *fn = nullptr;
+    cudaDriverEntryPointQueryResult qres;
+    if (!cuda_ok(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres)) || qres != cudaDriverEntryPointSuccess ||
+        fn == nullptr)
+        return SAL_E_LAUNCH;
+    g_encode_tiled = reinterpret_cast<TensorMapEncodeTiledFn>(fn);
+    return SAL_OK;
+}
+
+int sal_encode_planes(CUtensorMap *out, const void *bw, int K, int N, int q, int box_cols, int box_planes, int box_words) {
+    if (tensor_map_encoder() != SAL_OK) return SAL_E_LAUNCH;
+    // [K/32 words][q planes][N columns], innermost first; strides in bytes of all but the innermost dimension
+    const cuuint64_t dims[3] = {(cuuint64_t)N, (cuuint64_t)q, (cuuint64_t)(K / 32)};
+    const cuuint64_t strides[2] = {(cuuint64_t)N * 4, (cuuint64_t)N * 4 * (cuuint64_t)q};  // N % 4 == 0 keeps them multiples of 16
+    const cuuint32_t box[3] = {(cuuint32_t)box_cols, (cuuint32_t)box_planes, (cuuint32_t)box_words};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    const CUresult r = g_encode_tiled(out, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, const_cast<void *>(bw), dims, strides, box,
+                                      estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? SAL_OK : SAL_E_LAUNCH;
+}
+
+int sal_encode_rows(CUtensorMap *out, const void *base, int cols, int rows, int box_cols, int box_rows, int swizzle128) {
+    if (tensor_map_encoder() != SAL_OK) return SAL_E_LAUNCH;
+    const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+    const cuuint64_t strides[1] = {(cuuint64_t)cols * 2};   // callers: a multiple of 16
+    const cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
+    const cuuint32_t estr[2] = {1, 1};
+    const CUresult r = g_encode_tiled(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(base), dims, strides, box, estr,
+                                      CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? SAL_OK : SAL_E_LAUNCH;
+}
 
 // ------------------------------------------------------------------------------------------
 // C ABI
@@ -1913,6 +1969,8 @@ int sal_debug_set(const char *key, int value) {
     else if (eq("cost_r0")) g_cost_r0 = value / 1000.0;
     else if (eq("cost_r1")) g_cost_r1 = value / 1000.0;
     else if (eq("cost_rw")) g_cost_rw = value / 1000.0;
+    else if (eq("mma_min_rows")) g_mma_min_rows = value;
+    else if (eq("mma_min_rows_block")) g_mma_min_rows_block = value;
     else if (eq("cost_r1_acc")) g_cost_r1_acc = value / 1000.0;
     else return SAL_E_UNSUPPORTED;
     {
@@ -1956,8 +2014,10 @@ int sal_lutgemv_shift_scale(const void *bw, const void *alpha, const void *bias,
     rc = device_info(&dev);
     if (rc != SAL_OK) return rc;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    if (!(flags & SAL_FORCE_GENERIC) && tiled_eligible(bw, alpha, bias, x, y, M, K, N, q, num_groups)) {
-        sal_problem sp = {bw, alpha, bias, x, y, M, K, N, q, num_groups};
+    const sal_problem sp = {bw, alpha, bias, x, y, M, K, N, q, num_groups};
+    const bool tiled = tiled_eligible(bw, alpha, bias, x, y, M, K, N, q, num_groups);
+    if (mma_wanted(&sp, 1, flags, sal_mma::ROW, tiled)) return run_mma_group(&sp, 1, sal_mma::ROW, flags, workspace, workspace_bytes, s);
+    if (!(flags & SAL_FORCE_GENERIC) && tiled) {
         rc = run_tiled_group(&sp, 1, flags, workspace, workspace_bytes, s, nullptr);
         // a scratch buffer that is too small for this shape (or more row pairs x column ranges than it has
         // arrival counters) is not an error for the reference-style call: the generic kernel takes it
@@ -2020,8 +2080,12 @@ static int block_entry(int kind, const void *bw, const void *alpha, const void *
     p.gs = N / num_groups;
     p.num_apot = num_apot;
     p.accumulate = (flags & SAL_ACCUMULATE) ? 1 : 0;
-    if (!(flags & SAL_FORCE_GENERIC) && block_tiled_eligible(bw, alpha, x, M, K, N, q, num_groups, kind, num_apot)) {
-        sal_problem sp = {bw, alpha, bias, x, y, M, K, N, q, /*num_groups (unused in block mode)*/ 1};
+    const sal_problem sp = {bw, alpha, bias, x, y, M, K, N, q, num_groups};
+    const sal_mma::AlphaLayout layout = kind == B_F16 ? sal_mma::BLOCK_F16 : sal_mma::BLOCK_U16;
+    const bool tiled = block_tiled_eligible(bw, alpha, x, M, K, N, q, num_groups, kind, num_apot);
+    if (kind != B_I8 && mma_wanted(&sp, 1, flags, layout, tiled))
+        return run_mma_group(&sp, 1, layout, flags & (SAL_ACCUMULATE | SAL_PDL), workspace, workspace_bytes, reinterpret_cast<cudaStream_t>(stream));
+    if (!(flags & SAL_FORCE_GENERIC) && tiled) {
         const BlockAlpha blk = {kind, num_groups, N / num_groups, num_apot};
         rc = run_tiled_group(&sp, 1, flags & (SAL_ACCUMULATE | SAL_PDL), workspace, workspace_bytes,
                              reinterpret_cast<cudaStream_t>(stream), nullptr, nullptr, nullptr, &blk);
@@ -2049,9 +2113,25 @@ int sal_lutgemm_block_shift_int8(const void *bw, const void *alpha_i8, const voi
     return block_entry(B_I8, bw, alpha_i8, bias, x, y, M, K, N, q, num_groups, num_apot, flags, workspace, workspace_bytes, stream);
 }
 
+size_t sal_lutgemm_rows_workspace_bytes(int M) {
+    const int mt = M < 1 ? 1 : (M > 256 ? 256 : M);
+    return WS_PARTIAL_OFFSET + (size_t)148 * 2 * 128 * mt * sizeof(float);
+}
+
+int sal_lutgemm_rows(int alpha_layout, const void *bw, const void *alpha, const void *bias, const void *x, void *y, int M, int K, int N,
+                     int q, int num_groups, unsigned flags, void *workspace, size_t workspace_bytes, void *stream) {
+    int rc = validate_common(bw, alpha, x, y, M, K, N, q, sal_mma::MAX_ROWS);
+    if (rc != SAL_OK) return rc;
+    if (alpha_layout < 0 || alpha_layout > 2 || num_groups <= 0 || (alpha_layout == 0 ? K : N) % num_groups != 0) return SAL_E_SHAPE;
+    const sal_problem sp = {bw, alpha, bias, x, y, M, K, N, q, num_groups};
+    const sal_mma::AlphaLayout layout = static_cast<sal_mma::AlphaLayout>(alpha_layout);
+    if (!sal_mma::eligible(bw, alpha, x, M, K, N, q, num_groups, layout)) return SAL_E_UNSUPPORTED;
+    return run_mma_group(&sp, 1, layout, flags & (SAL_ACCUMULATE | SAL_PDL), workspace, workspace_bytes, reinterpret_cast<cudaStream_t>(stream));
+}
+
 int sal_lutgemv_grouped(const sal_problem *problems, int count, unsigned flags, void *workspace,
                         size_t workspace_bytes, void *stream) {
-    int rc = validate_grouped(problems, count, false);
+    int rc = validate_grouped(problems, count, flags, false);
     if (rc != SAL_OK) return rc;
     DeviceInfo *dev = nullptr;
     rc = device_info(&dev);
@@ -2061,6 +2141,14 @@ int sal_lutgemv_grouped(const sal_problem *problems, int count, unsigned flags, 
     int sizes[SAL_MAX_GROUP];
     const int nclass = split_by_q(problems, count, classes, sizes, nullptr);
     for (int c = 0; c < nclass; ++c) {
+        if (mma_wanted(classes[c], sizes[c], flags, sal_mma::ROW, true)) {
+            rc = run_mma_group(classes[c], sizes[c], sal_mma::ROW, flags, workspace, workspace_bytes, reinterpret_cast<cudaStream_t>(stream));
+            // a scratch buffer without room for silu(x) * x_mul: the two-row kernel forms it in its tables
+            if (rc == SAL_OK || rc != SAL_E_WORKSPACE || classes[c][0].M > SAL_MAX_M) {
+                if (rc != SAL_OK) return rc;
+                continue;
+            }
+        }
         rc = run_tiled_group(classes[c], sizes[c], flags, workspace, workspace_bytes, reinterpret_cast<cudaStream_t>(stream), nullptr);
         if (rc != SAL_OK) return rc;
     }
@@ -2070,7 +2158,7 @@ int sal_lutgemv_grouped(const sal_problem *problems, int count, unsigned flags, 
 int sal_lutgemv_grouped_exchange(const sal_problem *problems, int count, unsigned flags, void *workspace,
                                  size_t workspace_bytes, const sal_exchange *exchange, int *writers_out, void *stream) {
     if (!exchange) return SAL_E_NULL;
-    int rc = validate_grouped(problems, count, true);
+    int rc = validate_grouped(problems, count, flags, true);
     if (rc != SAL_OK) return rc;
     if (!exchange->gather_offsets) return SAL_E_NULL;
     DeviceInfo *dev = nullptr;
@@ -2101,14 +2189,16 @@ struct sal_prepared {
     int nlaunch;
     int writers;
     size_t ws_need;
+    bool on_mma[SAL_MAX_GROUP];   // class c is mma[c] (several rows), else launch[c]
     BuiltLaunch launch[SAL_MAX_GROUP];
+    sal_mma::Built mma[SAL_MAX_GROUP];
 };
 
 int sal_prepare_grouped(const sal_problem *problems, int count, unsigned flags, const sal_exchange *exchange,
                         sal_prepared **out) {
     if (!out) return SAL_E_NULL;
     *out = nullptr;
-    int rc = validate_grouped(problems, count, exchange != nullptr);
+    int rc = validate_grouped(problems, count, flags, exchange != nullptr);
     if (rc != SAL_OK) return rc;
     if (exchange && !exchange->gather_offsets) return SAL_E_NULL;
     DeviceInfo *dev = nullptr;
@@ -2128,6 +2218,18 @@ int sal_prepare_grouped(const sal_problem *problems, int count, unsigned flags, 
             ex = *exchange;
             ex.gather_offsets = offs;
             if (ex.slot < 0) ex.slot = 0;
+        }
+        if (!exchange && mma_wanted(classes[c], sizes[c], flags, sal_mma::ROW, true)) {
+            h->on_mma[c] = true;
+            rc = sal_mma::build(classes[c], sizes[c], sal_mma::ROW, flags, (size_t)1 << 40, dev->sms, &h->mma[c]);
+            if (rc != SAL_OK) {
+                delete h;
+                return rc;
+            }
+            for (int i = 0; i < sizes[c]; ++i) h->writers += (classes[c][i].N + 255) / 256;
+            const size_t need = sal_mma::scratch_bytes(h->mma[c]);
+            if (need > h->ws_need) h->ws_need = need;
+            continue;
         }
         rc = build_tiled_group(classes[c], sizes[c], flags, true, true, exchange ? &ex : nullptr, nullptr, &h->launch[c]);
         if (rc != SAL_OK) {
@@ -2150,7 +2252,8 @@ int sal_launch_prepared(const sal_prepared *prepared, void *workspace, size_t wo
     int dev = -1;
     if (!cuda_ok(cudaGetDevice(&dev)) || dev != prepared->device) return SAL_E_DEVICE;
     for (int c = 0; c < prepared->nlaunch; ++c) {
-        const int rc = launch_built(prepared->launch[c], workspace, workspace_bytes, slot, reinterpret_cast<cudaStream_t>(stream));
+        const int rc = prepared->on_mma[c] ? sal_mma::launch(prepared->mma[c], workspace, workspace_bytes, reinterpret_cast<cudaStream_t>(stream))
+                                           : launch_built(prepared->launch[c], workspace, workspace_bytes, slot, reinterpret_cast<cudaStream_t>(stream));
         if (rc != SAL_OK) return rc;
     }
     return SAL_OK;

@@ -201,14 +201,15 @@ class GroupedLaunch:
     storage must stay where it is.  Problems may differ in ``nb`` (mixed precision): the launch is
     then one kernel per distinct plane count."""
 
-    def __init__(self, problems, *, pdl=False, accumulate=False, atomic_fixed=False, swiglu_fixed=False, exchange=None):
+    def __init__(self, problems, *, pdl=False, accumulate=False, atomic_fixed=False, swiglu_fixed=False, exchange=None, many_rows=False):
         self._lib = _lib.load()
         self._arr, self._keep = marshal_problems(problems, atomic_fixed=atomic_fixed, swiglu_fixed=swiglu_fixed)
         self._device = problems[0]["output"].device
         if self._device.index is None:
             self._device = torch.device("cuda", torch.cuda.current_device())
         self._flags = ((_lib.SAL_PDL if pdl else 0) | (_lib.SAL_ACCUMULATE if accumulate else 0)
-                       | (_lib.SAL_OUT_FIXED_ATOMIC if atomic_fixed else 0) | (_lib.SAL_SWIGLU_FIXED if swiglu_fixed else 0))
+                       | (_lib.SAL_OUT_FIXED_ATOMIC if atomic_fixed else 0) | (_lib.SAL_SWIGLU_FIXED if swiglu_fixed else 0)
+                       | (_lib.SAL_MANY_ROWS if many_rows else 0))
         self._exchange = exchange          # a ctypes SalExchange (and what it points to), or None
         handle = _lib._vp()
         with torch.cuda.device(self._device):
@@ -275,7 +276,7 @@ def prepare_grouped(problems, **kwargs) -> GroupedLaunch:
     return GroupedLaunch(problems, **kwargs)
 
 
-def lutgemv_grouped(problems, *, pdl=False, accumulate=False, atomic_fixed=False, swiglu_fixed=False):
+def lutgemv_grouped(problems, *, pdl=False, accumulate=False, atomic_fixed=False, swiglu_fixed=False, many_rows=False):
     """Several independent mode-A products in one launch.  ``problems`` is a list
     of dicts with keys output, bWeight, alpha, bias (or None), d_input,
     mSize, kSize, nb, num_groups and optionally d_input_mul (the activation is then
@@ -284,8 +285,9 @@ def lutgemv_grouped(problems, *, pdl=False, accumulate=False, atomic_fixed=False
     ``atomic_fixed=True``: every ``output`` is an int64 fixed-point accumulator (units of 2**-32, see
     :data:`FIXED_ONE`) the product is ADDED to with integer atomics: no split-K reduction tail, and — integer
     sums being independent of the order of arrival — still bit-identical from run to run.
-    ``swiglu_fixed=True``: d_input and d_input_mul are such accumulators."""
-    GroupedLaunch(problems, pdl=pdl, accumulate=accumulate, atomic_fixed=atomic_fixed, swiglu_fixed=swiglu_fixed)()
+    ``swiglu_fixed=True``: d_input and d_input_mul are such accumulators.
+    ``many_rows=True``: up to ``SAL_MAX_ROWS`` rows (shapes of the tensor-core product) instead of ``SAL_MAX_M``."""
+    GroupedLaunch(problems, pdl=pdl, accumulate=accumulate, atomic_fixed=atomic_fixed, swiglu_fixed=swiglu_fixed, many_rows=many_rows)()
 
 
 def compiled_module():

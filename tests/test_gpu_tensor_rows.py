@@ -1,0 +1,120 @@
+"""Several activation rows on the tensor cores (csrc/sal_mma.cu) where the kernel's edges are: column tiles of 128, row tiles of up to
+256 padded to 16, units of 128 and steps of 64 features, groups that straddle a unit, planes fetched by TMA or by 4-byte copies, a tile
+shared by many CTAs or none, and the scratch limits that change the split.
+
+Reference: the same product in float64.  Bound per element: the output's fp16 rounding (2**-11 of the value, or half the smallest
+subnormal) plus one fp32 rounding (2**-23, which also covers truncation) per accumulation step, of which a tile has K * q / 16 and the
+sum over CTAs at most 64, each of at most the sum of the magnitudes."""
+import pytest
+import torch
+
+from shiftaddllm_b200 import _lib, lutgemm
+from shiftaddllm_b200.quant import LutLinear
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(layout, m, k, n, q, g, seed=0):
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    bits = torch.randint(-2 ** 31, 2 ** 31, (k // 32, q, n), dtype=torch.int32, device="cuda", generator=gen)
+    shape = (k // g, q, n) if layout == 0 else (k // 8, q, n // g)
+    if layout == 2:
+        alpha = torch.randint(0, 512, shape, device="cuda", generator=gen).to(torch.int16)
+        mult = sum(torch.exp2(((alpha >> s) & 7).double()) for s in (0, 3, 6))
+    else:
+        alpha = (torch.exp2(-torch.randint(2, 9, shape, device="cuda", generator=gen).float())
+                 * (0.5 + 0.5 * torch.rand(shape, device="cuda", generator=gen))).half()
+        mult = alpha.double()
+    x = torch.randn(m, k, device="cuda", generator=gen).half()
+    bias = (0.1 * torch.randn(n, device="cuda", generator=gen)).half()
+    return bits, alpha, mult, x, bias
+
+
+def _reference(bits, mult, x, bias):
+    words, q, n = bits.shape
+    signs = ((bits[:, None] >> torch.arange(32, device="cuda", dtype=torch.int32).view(1, 32, 1, 1)) & 1).reshape(32 * words, q, n).double() * 2 - 1
+    scale = mult.repeat_interleave(32 * words // mult.shape[0], 0).repeat_interleave(n // mult.shape[2], 2)
+    y = x.double() @ (signs * scale).sum(1) + bias.double()
+    size = x.double().abs() @ scale.sum(1) + bias.double().abs()
+    bound = 2.0 ** -11 * y.abs() + 2.0 ** -25 + (32 * words * q / 16 + 64) * 2.0 ** -23 * size
+    return y, bound
+
+
+def _call(layout, bits, alpha, x, bias, y, groups, ws, ws_bytes, flags=0):
+    return _lib.load().sal_lutgemm_rows(layout, bits.data_ptr(), alpha.data_ptr(), bias.data_ptr(), x.data_ptr(), y.data_ptr(), x.shape[0],
+                                        x.shape[1], bits.shape[2], bits.shape[1], groups, flags, ws.data_ptr() if ws_bytes else None, ws_bytes,
+                                        torch.cuda.current_stream().cuda_stream)
+
+
+# layout, rows, K, N, q, group; scratch bytes (None: what the header asks for)
+CASES = [
+    (0, 2, 32, 8, 1, 32, None), (0, 16, 64, 128, 2, 64, None), (0, 17, 96, 132, 3, 96, None), (0, 3, 2080, 1378, 3, 32, None),
+    (0, 64, 1024, 1000, 4, 128, None), (0, 65, 128, 127, 3, 128, None), (0, 255, 512, 256, 3, 256, None), (0, 257, 384, 260, 2, 128, None),
+    (0, 600, 256, 64, 3, 256, None), (0, 8, 160, 130, 3, 160, None), (0, 5, 11008, 16, 3, 128, None), (0, 1, 256, 256, 3, 128, None),
+    (1, 2, 64, 16, 3, 16, None), (1, 33, 288, 96, 4, 32, None), (1, 9, 256, 144, 2, 48, None), (1, 130, 512, 512, 3, 256, None),
+    (1, 1, 32, 128, 1, 128, None), (2, 12, 256, 256, 3, 16, None), (2, 70, 96, 80, 2, 16, None),
+    (0, 16, 4096, 512, 3, 128, 0), (0, 16, 4096, 512, 3, 128, 16384 + 3 * 1024 * 16), (1, 40, 2048, 384, 2, 16, 0),
+]
+
+
+@pytest.mark.parametrize("layout,m,k,n,q,g,scratch", CASES)
+def test_rows_against_float64(layout, m, k, n, q, g, scratch):
+    bits, alpha, mult, x, bias = _case(layout, m, k, n, q, g)
+    groups = k // g if layout == 0 else n // g
+    ref, bound = _reference(bits, mult, x, bias)
+    need = _lib.load().sal_lutgemm_rows_workspace_bytes(m) if scratch is None else scratch
+    ws = torch.zeros(max(need, 256), dtype=torch.uint8, device="cuda")
+    y = torch.full((m, n), float("nan"), dtype=torch.float16, device="cuda")
+    for rep in range(2):   # the second call finds the scratch buffer as the first one left it
+        assert _call(layout, bits, alpha, x, bias, y, groups, ws, need) == 0
+        assert ((y.double() - ref).abs() <= bound).all(), rep
+    first = y.clone()
+    assert _call(layout, bits, alpha, x, bias, y, groups, ws, need, _lib.SAL_ACCUMULATE) == 0
+    assert ((y.double() - ref - first.double()).abs() <= bound + 2.0 ** -11 * (ref + first.double()).abs()).all()
+    if need >= 256:
+        assert _lib.load().sal_workspace_status(ws.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+
+
+def test_layer_of_many_rows_and_its_limits():
+    """LutLinear takes any number of rows; rows beyond one call's limit go in further calls, and what the tensor-core product does not
+    take (more than four planes) still runs 64 rows at a time."""
+    for q, rows in ((3, 4100), (5, 130)):
+        bits, alpha, mult, x, bias = _case(0, rows, 256, 64, q, 128, seed=q)
+        lin = LutLinear(256, 64, 128, q, bias=bias)
+        lin.binaryWeight = bits
+        lin.set_row_alpha(alpha)
+        ref, bound = _reference(bits, mult, x, bias)
+        assert ((lin(x).double() - ref).abs() <= bound).all()
+        wide = lin(x.float().view(2, rows // 2, 256))
+        assert wide.dtype == torch.float32 and wide.shape == (2, rows // 2, 64)
+    lib, y = _lib.load(), torch.empty(64, 64, dtype=torch.float16, device="cuda")
+    ws = torch.zeros(lutgemm.workspace_for(y.device, 64, 64).numel(), dtype=torch.uint8, device="cuda")
+    args = (_case(0, 64, 256, 64, 5, 128))
+    assert _call(0, args[0], args[1], args[3], args[4], y, 2, ws, ws.numel()) == _lib.SAL_E_UNSUPPORTED
+    assert lib.sal_lutgemm_rows(0, args[0].data_ptr(), args[1].data_ptr(), None, args[3].data_ptr(), y.data_ptr(), 4097, 256, 64, 4, 2, 0,
+                                None, 0, None) == _lib.SAL_E_SHAPE
+
+
+@pytest.mark.parametrize("m", [7, 64, 300])   # from 7 rows on
+def test_grouped_rows_with_swiglu(m):
+    """Problems of different widths in one launch, and the activation silu(x) * x_mul of a down projection."""
+    probs, refs = [], []
+    for i, (k, n) in enumerate(((256, 264), (512, 128), (256, 1000))):
+        bits, alpha, mult, x, bias = _case(0, m, k, n, 3, 128, seed=i)
+        y = torch.empty(m, n, dtype=torch.float16, device="cuda")
+        probs.append(dict(output=y, bWeight=bits, alpha=alpha, bias=bias, d_input=x, mSize=n, kSize=k, nb=3, num_groups=k // 128))
+        refs.append(_reference(bits, mult, x, bias))
+    lutgemm.lutgemv_grouped(probs, pdl=True, many_rows=m > 64)
+    for p, (ref, bound) in zip(probs, refs):
+        assert ((p["output"].double() - ref).abs() <= bound).all()
+    if m > 64:
+        with pytest.raises(RuntimeError):
+            lutgemm.lutgemv_grouped(probs)
+    p = probs[1]
+    p["d_input_mul"] = torch.randn(m, 512, device="cuda", generator=torch.Generator(device="cuda").manual_seed(9)).half()
+    lutgemm.lutgemv_grouped([p], pdl=True, many_rows=m > 64)
+    act = torch.nn.functional.silu(p["d_input"]) * p["d_input_mul"]
+    bits, alpha, mult, _, bias = _case(0, m, 512, 128, 3, 128, seed=1)
+    ref, bound = _reference(bits, mult, act, bias)
+    # silu is rounded to fp16 before the product here and in torch; a last-bit difference of its exponential moves an activation by 2**-10
+    assert ((p["output"].double() - ref).abs() <= bound + 2.0 ** -10 * (act.double().abs() @ mult.sum(1).repeat_interleave(128, 0))).all()
