@@ -100,6 +100,15 @@ int sal_greedy_token_f16(const void *logits_f16, void *logits_f32, int vocab, in
 /* out = silu(gate) * up, fp16 vectors of n elements. */
 int sal_silu_mul_f16(const void *gate, const void *up, void *out, int n, void *stream);
 
+/* A prompt's rows between its products.
+ * sal_rope_rows_f16: rows 0..m-1 at positions pos0, pos0 + 1, ..: q [m][heads][hd] is rotated in place, k [m][kv_heads][hd]
+ * rotated and v copied into the cache rows.  hd a multiple of 16, all of them 16-byte aligned.
+ * sal_causal_softmax_f16: scores [heads][m][T] (unscaled, fp16) become probabilities in place; row i sees the positions
+ * 0 .. first + i, the others become 0.  Sums in fp32. */
+int sal_rope_rows_f16(void *q, const void *k, const void *v, const void *cos, const void *sin, int pos0, int m, void *k_cache, void *v_cache,
+                      int heads, int kv_heads, int hd, int max_len, void *stream);
+int sal_causal_softmax_f16(void *scores, int heads, int m, int T, int first, float scale, void *stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -414,6 +414,99 @@ __global__ void silu_mul_kernel(const __half *gate, const __half *up, __half *ou
     }
 }
 
+// The same, eight elements per thread (n and the pointers allow 16-byte accesses): a prompt's rows are tens of MB.
+__global__ void __launch_bounds__(256) silu_mul_vec_kernel(const uint4 *gate, const uint4 *up, uint4 *out, int n8) {
+    pdl_prologue();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n8) return;
+    const uint4 gv = gate[i], uv = up[i];
+    uint4 ov;
+    const __half *gh = reinterpret_cast<const __half *>(&gv), *uh = reinterpret_cast<const __half *>(&uv);
+    __half *oh = reinterpret_cast<__half *>(&ov);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const float g = __half2float(gh[k]);
+        oh[k] = __float2half_rn(__half2float(__float2half_rn(g / (1.f + __expf(-g)))) * __half2float(uh[k]));
+    }
+    out[i] = ov;
+}
+
+// Rotary step of `m` prompt rows at positions pos0, pos0 + 1, ..: q is rotated in place, the rotated keys and the values go to the
+// cache rows.  A thread takes eight feature pairs (16-byte accesses): q heads first, then k heads, then the value copy.
+__global__ void __launch_bounds__(256) rope_rows_kernel(__half *q, const __half *k, const __half *v, const float *cos_t, const float *sin_t,
+                                                        int pos0, __half *k_cache, __half *v_cache, int heads, int kv_heads, int hd) {
+    pdl_prologue();
+    const int row = blockIdx.y, pos = pos0 + row, half = hd / 2, h8 = half / 8;
+    const int idx = blockIdx.x * blockDim.x + threadIdx.x, nq = heads * h8, nk = kv_heads * h8, nv = kv_heads * hd / 8;
+    if (idx < nq + nk) {
+        const bool is_q = idx < nq;
+        const int j = is_q ? idx : idx - nq, h = j / h8, i = (j % h8) * 8;
+        const __half *src = is_q ? q + (size_t)row * heads * hd : k + (size_t)row * kv_heads * hd;
+        __half *dst = is_q ? q + (size_t)row * heads * hd : k_cache + (size_t)pos * kv_heads * hd;
+        const uint4 av = *reinterpret_cast<const uint4 *>(src + h * hd + i), bv = *reinterpret_cast<const uint4 *>(src + h * hd + half + i);
+        const __half *ah = reinterpret_cast<const __half *>(&av), *bh = reinterpret_cast<const __half *>(&bv);
+        uint4 ra, rb;
+        __half *rah = reinterpret_cast<__half *>(&ra), *rbh = reinterpret_cast<__half *>(&rb);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const float c = cos_t[(size_t)pos * half + i + e], s = sin_t[(size_t)pos * half + i + e];
+            const float a = __half2float(ah[e]), b = __half2float(bh[e]);
+            rah[e] = __float2half_rn(a * c - b * s);
+            rbh[e] = __float2half_rn(b * c + a * s);
+        }
+        *reinterpret_cast<uint4 *>(dst + h * hd + i) = ra;
+        *reinterpret_cast<uint4 *>(dst + h * hd + half + i) = rb;
+    } else if (idx < nq + nk + nv) {
+        const int j = (idx - nq - nk) * 8;
+        *reinterpret_cast<uint4 *>(v_cache + (size_t)pos * kv_heads * hd + j) = *reinterpret_cast<const uint4 *>(v + (size_t)row * kv_heads * hd + j);
+    }
+}
+
+// Causal softmax of a prompt's attention scores, in place: scores fp16 [heads][m][T] (unscaled), row i sees positions 0 .. first + i.
+// One warp per row: a running maximum and sum over the visible part in fp32, then the probabilities (rounded to fp16, as the product
+// with the values takes them) and zeros behind it.  Bound by its two reads and one write; the operators it replaces (to fp32, scale,
+// mask, softmax, to fp16) moved the fp32 scores four times.
+template <int VEC>
+__global__ void __launch_bounds__(128) causal_softmax_kernel(__half *scores, int rows, int m, int T, int first, float scale) {
+    pdl_prologue();
+    const int r = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (r >= rows) return;
+    __half *p = scores + (size_t)r * T;
+    const int vis = min(first + r % m + 1, T);
+    float mx = -INFINITY, sum = 0.f;
+    for (int t = lane * VEC; t < vis; t += 32 * VEC) {
+        __half h[VEC];
+        if (VEC == 8) *reinterpret_cast<uint4 *>(h) = *reinterpret_cast<const uint4 *>(p + t);
+        else h[0] = p[t];
+        float f[VEC], lm = -INFINITY;
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) {
+            f[e] = t + e < vis ? __half2float(h[e]) * scale : -INFINITY;
+            lm = fmaxf(lm, f[e]);
+        }
+        const float nm = fmaxf(mx, lm);   // drops NaN scores; the sum keeps them
+        float part = 0.f;
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) part += f[e] == -INFINITY ? 0.f : __expf(f[e] - nm);
+        sum = (sum == 0.f ? 0.f : sum * __expf(mx - nm)) + part;
+        mx = nm;
+    }
+    const float m_all = warp_max(mx);
+    sum = warp_sum(sum == 0.f ? 0.f : sum * __expf(mx - m_all));
+    for (int t = lane * VEC; t < T; t += 32 * VEC) {
+        __half h[VEC];
+        if (t < vis) {
+            if (VEC == 8) *reinterpret_cast<uint4 *>(h) = *reinterpret_cast<const uint4 *>(p + t);
+            else h[0] = p[t];
+        }
+#pragma unroll
+        for (int e = 0; e < VEC; ++e)
+            h[e] = t + e < vis ? __float2half_rn(__expf(__half2float(h[e]) * scale - m_all) / sum) : __float2half_rn(0.f);
+        if (VEC == 8) *reinterpret_cast<uint4 *>(p + t) = *reinterpret_cast<const uint4 *>(h);
+        else p[t] = h[0];
+    }
+}
+
 // All helpers are launched with the programmatic-stream-serialization attribute (see pdl_prologue).
 template <typename... KArgs, typename... Args>
 int launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, void *stream, Args... args) {
@@ -1093,8 +1186,35 @@ int sal_greedy_token_f16(const void *logits_f16, void *logits_f32, int vocab, in
 int sal_silu_mul_f16(const void *gate, const void *up, void *out, int n, void *stream) {
     if (!gate || !up || !out) return SAL_E_NULL;
     if (n < 1) return SAL_E_SHAPE;
+    if (n % 8 == 0 && ((reinterpret_cast<uintptr_t>(gate) | reinterpret_cast<uintptr_t>(up) | reinterpret_cast<uintptr_t>(out)) & 15) == 0)
+        return launch_pdl(silu_mul_vec_kernel, dim3((n / 8 + 255) / 256), dim3(256), 0, stream, reinterpret_cast<const uint4 *>(gate),
+                          reinterpret_cast<const uint4 *>(up), reinterpret_cast<uint4 *>(out), n / 8);
     return launch_pdl(silu_mul_kernel, dim3((n + 255) / 256), dim3(256), 0, stream, reinterpret_cast<const __half *>(gate),
                       reinterpret_cast<const __half *>(up), reinterpret_cast<__half *>(out), n);
+}
+
+int sal_rope_rows_f16(void *q, const void *k, const void *v, const void *cos, const void *sin, int pos0, int m, void *k_cache, void *v_cache,
+                      int heads, int kv_heads, int hd, int max_len, void *stream) {
+    if (!q || !k || !v || !cos || !sin || !k_cache || !v_cache) return SAL_E_NULL;
+    if (heads < 1 || kv_heads < 1 || hd < 16 || hd % 16 || m < 1 || m > 65535 || pos0 < 0 || pos0 > max_len - m) return SAL_E_SHAPE;
+    if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(k_cache) |
+         reinterpret_cast<uintptr_t>(v_cache)) & 15)
+        return SAL_E_ALIGN;
+    const int total = (heads + kv_heads) * (hd / 16) + kv_heads * (hd / 8);
+    return launch_pdl(rope_rows_kernel, dim3((total + 255) / 256, m), dim3(256), 0, stream, reinterpret_cast<__half *>(q),
+                      reinterpret_cast<const __half *>(k), reinterpret_cast<const __half *>(v), reinterpret_cast<const float *>(cos),
+                      reinterpret_cast<const float *>(sin), pos0, reinterpret_cast<__half *>(k_cache), reinterpret_cast<__half *>(v_cache), heads,
+                      kv_heads, hd);
+}
+
+int sal_causal_softmax_f16(void *scores, int heads, int m, int T, int first, float scale, void *stream) {
+    if (!scores) return SAL_E_NULL;
+    if (heads < 1 || m < 1 || T < 1 || first < 0 || (long long)heads * m > 0x3fffffff) return SAL_E_SHAPE;
+    const int rows = heads * m;
+    __half *p = reinterpret_cast<__half *>(scores);
+    if (T % 8 == 0 && (reinterpret_cast<uintptr_t>(scores) & 15) == 0)
+        return launch_pdl(causal_softmax_kernel<8>, dim3((rows + 3) / 4), dim3(128), 0, stream, p, rows, m, T, first, scale);
+    return launch_pdl(causal_softmax_kernel<1>, dim3((rows + 3) / 4), dim3(128), 0, stream, p, rows, m, T, first, scale);
 }
 
 }  // extern "C"

@@ -131,3 +131,22 @@ def silu_mul(gate, up, out):
     lib = _lib.load()
     _lib.check(lib.sal_silu_mul_f16(gate.data_ptr(), up.data_ptr(), out.data_ptr(), gate.numel(), _stream(gate)),
                "sal_silu_mul_f16")
+
+
+def rope_rows(q, k, v, cos, sin, pos0: int, k_cache, v_cache, heads, kv_heads, hd) -> bool:
+    """Rotary step of a prompt's rows at positions pos0, pos0 + 1, ..: q [m, heads * hd] in place, keys and values into the cache rows.
+    False where the helper does not take the shape (nothing is launched then)."""
+    lib = _lib.load()
+    rc = lib.sal_rope_rows_f16(q.data_ptr(), k.data_ptr(), v.data_ptr(), cos.data_ptr(), sin.data_ptr(), int(pos0), q.shape[0],
+                               k_cache.data_ptr(), v_cache.data_ptr(), heads, kv_heads, hd, k_cache.shape[0], _stream(q))
+    if rc in (_lib.SAL_E_SHAPE, _lib.SAL_E_ALIGN):
+        return False
+    _lib.check(rc, "sal_rope_rows_f16")
+    return True
+
+
+def causal_softmax(scores, first: int, scale: float):
+    """scores fp16 [heads, m, T] -> probabilities, in place; row i sees positions 0 .. first + i."""
+    lib = _lib.load()
+    _lib.check(lib.sal_causal_softmax_f16(scores.data_ptr(), scores.shape[0], scores.shape[1], scores.shape[2], int(first), float(scale),
+                                          _stream(scores)), "sal_causal_softmax_f16")

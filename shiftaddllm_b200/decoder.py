@@ -78,12 +78,12 @@ class _Block:
                 "gate_proj": self.gate_proj, "up_proj": self.up_proj, "down_proj": self.down_proj}
 
 
-def _group(lins, x, outs, pdl=True, x_mul=None, atomic=False, swiglu_fixed=False):
+def _group(lins, x, outs, pdl=True, x_mul=None, atomic=False, swiglu_fixed=False, many_rows=False):
     """One grouped LUT-GEMV launch: every layer of `lins` applied to the same activation row
     (`x_mul` given: to silu(x) * x_mul, formed inside the kernel)."""
     probs = [dict(output=o, bWeight=l.binaryWeight, alpha=l.alpha, bias=l.bias, d_input=x, mSize=l.N, kSize=l.K,
                   nb=l.wbit, num_groups=l.alpha.shape[0], d_input_mul=x_mul) for l, o in zip(lins, outs)]
-    lutgemm.lutgemv_grouped(probs, pdl=pdl, atomic_fixed=atomic, swiglu_fixed=swiglu_fixed)
+    lutgemm.lutgemv_grouped(probs, pdl=pdl, atomic_fixed=atomic, swiglu_fixed=swiglu_fixed, many_rows=many_rows)
 
 
 class BcqLlamaDecoder:
@@ -285,11 +285,14 @@ class BcqLlamaDecoder:
             self.token.fill_(int(t))
             run()
 
+    PREFILL_ROWS = 512   # prompt rows of one pass (`prefill`): two full row tiles of the tensor-core product
+
     def prefill(self, token_ids, chunk: int = 64):
-        """Chunked prompt pass: rows of a chunk share each weight stream (M = chunk rows per product,
-        2 <= M <= 64; a last chunk of one token runs the M = 1 kernel).  RMSNorm, RoPE and the causal attention
-        over the cache are torch ops here (a prompt is processed once; the per-token step is where the fused
-        helpers matter).  Leaves the cache, `pos`, the logits of the last prompt token and the greedy next token
+        """Prompt pass: the rows of a pass share each weight stream (one product per layer and pass; a last pass of one
+        token runs the M = 1 kernel).  `chunk` below 64 bounds the rows of a pass; from 64 on passes of
+        up to PREFILL_ROWS are taken where the layers allow it (the result does not depend on it beyond rounding).  Between the
+        products: residual + RMSNorm, rotary step + cache write and causal softmax are one helper launch each, the two attention
+        products torch's batched matmul.  Leaves the cache, `pos`, the logits of the last prompt token and the greedy next token
         exactly where a token-by-token `feed` would."""
         s = self.shape
         hd, kvh, rep, h = s.head_dim, s.kv_heads, s.heads // s.kv_heads, s.hidden
@@ -298,46 +301,66 @@ class BcqLlamaDecoder:
         p0 = int(self.pos.item())
         if p0 + ids.numel() > self.max_len:
             raise ValueError("prompt does not fit the KV cache")
+        many = chunk == 64 and all(l.wbit <= 4 for b in self.blocks for l in b.linears().values())
+        rows = self.PREFILL_ROWS if many else chunk
         f16 = dict(dtype=torch.float16, device=self.device)
-        for c0 in range(0, ids.numel(), chunk):
-            tok = ids[c0:c0 + chunk]
-            m = tok.numel()
-            pos = torch.arange(p0 + c0, p0 + c0 + m, device=self.device)
-            total = p0 + c0 + m                                            # cached positions after this chunk
-            cos, sin = self.cos.index_select(0, pos)[:, None, :], self.sin.index_select(0, pos)[:, None, :]   # [m, 1, hd/2]
-
-            def rope(t, heads):
-                t = t.view(m, heads, 2, hd // 2).float()                   # rotate-half convention
-                a, b = t[:, :, 0, :], t[:, :, 1, :]
-                return torch.stack((a * cos - b * sin, b * cos + a * sin), dim=2).view(m, heads, hd).half()
-
-            causal = (torch.arange(total, device=self.device)[None, :] > pos[:, None]).view(1, m, 1, total)
+        scale = 1.0 / math.sqrt(hd)
+        for c0 in range(0, ids.numel(), rows):
+            tok = ids[c0:c0 + rows]
+            m, first = tok.numel(), p0 + c0
+            total = first + m                                              # cached positions after this pass
             x = self.embed.index_select(0, tok)                            # [m, hidden]
             q, k, v = torch.empty(m, h, **f16), torch.empty(m, kvh * hd, **f16), torch.empty(m, kvh * hd, **f16)
+            hn, attn, delta = torch.empty(m, h, **f16), torch.empty(m, h, **f16), None
             o_out, down = torch.empty(m, h, **f16), torch.empty(m, h, **f16)
             gate, up = torch.empty(m, s.ffn, **f16), torch.empty(m, s.ffn, **f16)
+            scores = torch.empty(s.heads, m, total, **f16)
+            qh, ah = q.view(m, s.heads, hd).transpose(0, 1), attn.view(m, s.heads, hd).transpose(0, 1)
             for li, blk in enumerate(self.blocks):
-                hn = F.rms_norm(x, (h,), blk.input_norm, s.eps)
-                _group((blk.q_proj, blk.k_proj, blk.v_proj), hn, (q, k, v))
-                qh, kh = rope(q, s.heads), rope(k, kvh)
-                self.k_cache[li].index_copy_(0, pos, kh)
-                self.v_cache[li].index_copy_(0, pos, v.view(m, kvh, hd))
+                self._prefill_norm(x, delta, blk.input_norm, hn)
+                _group((blk.q_proj, blk.k_proj, blk.v_proj), hn, (q, k, v), many_rows=many)
+                if not decode_ops.rope_rows(q, k, v, self.cos, self.sin, first, self.k_cache[li], self.v_cache[li], s.heads, kvh, hd):
+                    self._prefill_rope(q, k, v, first, li)
                 keys = self.k_cache[li, :total].permute(1, 2, 0)           # [kvh, hd, T]
-                vals = self.v_cache[li, :total].permute(1, 0, 2)           # [kvh, T, hd]
-                scores = torch.matmul(qh.view(m, kvh, rep, hd).permute(1, 0, 2, 3), keys[:, None]).float() * (1.0 / math.sqrt(hd))
-                scores = scores.masked_fill(causal, float("-inf"))         # [kvh, m, rep, T]
-                attn = torch.matmul(torch.softmax(scores, dim=-1).half(), vals[:, None])       # [kvh, m, rep, hd]
-                attn = attn.permute(1, 0, 2, 3).reshape(m, h).contiguous()
-                _group((blk.o_proj,), attn, (o_out,))
-                x = x + o_out
-                hn = F.rms_norm(x, (h,), blk.post_norm, s.eps)
-                _group((blk.gate_proj, blk.up_proj), hn, (gate, up))
-                _group((blk.down_proj,), gate, (down,), x_mul=up)          # SiLU(gate)*up formed in the table build
-                x = x + down
+                vals = self.v_cache[li, :total].transpose(0, 1)            # [kvh, T, hd]
+                if rep > 1:
+                    keys, vals = keys.repeat_interleave(rep, dim=0), vals.repeat_interleave(rep, dim=0)
+                torch.bmm(qh, keys, out=scores)
+                decode_ops.causal_softmax(scores, first, scale)
+                torch.bmm(scores, vals, out=ah)
+                _group((blk.o_proj,), attn, (o_out,), many_rows=many)
+                self._prefill_norm(x, o_out, blk.post_norm, hn)
+                _group((blk.gate_proj, blk.up_proj), hn, (gate, up), many_rows=many)
+                _group((blk.down_proj,), gate, (down,), x_mul=up, many_rows=many)   # with SiLU(gate)*up as its activation
+                delta = down
+            x = x + down
         hn = F.rms_norm(x[-1:], (h,), self.final_norm, s.eps)
         self.logits.copy_(torch.matmul(hn, self.lm_head.t()).float().view(-1))
         self.token.copy_(self.logits.argmax().view(1))
         self.pos.add_(ids.numel())
+
+    def _prefill_norm(self, x, delta, weight, out):
+        """x += delta (None: the first norm of a pass); out = rmsnorm(x) * weight."""
+        if x.shape[1] <= 12000:
+            decode_ops.residual_rmsnorm_rows(x, delta, weight, out, x, self.shape.eps)
+            return
+        if delta is not None:
+            x.add_(delta)
+        out.copy_(F.rms_norm(x, (x.shape[1],), weight, self.shape.eps))
+
+    def _prefill_rope(self, q, k, v, first, li):
+        """Head sizes the rotary helper does not take."""
+        s, m = self.shape, q.shape[0]
+        hd, kvh = s.head_dim, s.kv_heads
+        cos, sin = self.cos[first:first + m, None, :], self.sin[first:first + m, None, :]      # [m, 1, hd/2]
+
+        def rope(t, heads):
+            a, b = t.view(m, heads, 2, hd // 2).float().unbind(2)          # rotate-half convention
+            return torch.stack((a * cos - b * sin, b * cos + a * sin), dim=2).view(m, heads, hd).half()
+
+        self.k_cache[li, first:first + m] = rope(k, kvh)
+        self.v_cache[li, first:first + m] = v.view(m, kvh, hd)
+        q.copy_(rope(q, s.heads).view(m, -1))
 
     def generate(self, n):
         run = self.graph.replay if self.graph is not None else self.step
