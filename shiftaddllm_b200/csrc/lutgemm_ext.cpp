@@ -14,6 +14,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 
+#include <algorithm>
 #include <map>
 #include <mutex>
 #include <string>
@@ -163,6 +164,83 @@ void lutgemv_fused(torch::Tensor output, torch::Tensor bWeight, torch::Tensor al
                  "lutgemv_fused");
 }
 
+// LutLinear.forward in one call: input to fp16 rows, output allocated, the product of all rows (a tensor-core launch takes
+// SAL_MAX_ROWS of them, the others SAL_MAX_M) with the bias fused, result in the input's type and shape.  A layer of one token is a
+// few microseconds of GPU work; the same steps in Python (checks, stream and scratch look-ups, a call through ctypes) cost about 35.
+torch::Tensor lut_linear(const torch::Tensor &x, const torch::Tensor &bWeight, const torch::Tensor &alpha, const c10::optional<torch::Tensor> &bias,
+                         int64_t K, int64_t N, int64_t q, bool row_layout) {
+    TORCH_CHECK(x.dim() >= 1 && x.size(-1) == K, "last dim of the input must be ", K, ", got ", x.dim() ? x.size(-1) : 0);
+    TORCH_CHECK(x.is_cuda(), "d_input must be a CUDA tensor (there is no CPU path)");
+    TORCH_CHECK(K > 0 && N > 0 && q > 0 && K % 32 == 0, "in and out features and bits must be positive, in features a multiple of 32");
+    require(bWeight, torch::kInt32, "bWeight");
+    TORCH_CHECK(bWeight.numel() == (K / 32) * q * N, "bWeight must hold (kSize/32)*nb*mSize = ", (K / 32) * q * N, " words, has ", bWeight.numel());
+    const auto dev = x.device();
+    TORCH_CHECK(bWeight.device() == dev && alpha.device() == dev, "all tensors must live on the same device");
+    const auto kind = alpha.scalar_type();
+    int64_t groups = 0, per = 1, numel = 0;
+    if (kind == torch::kFloat16 && row_layout) {
+        TORCH_CHECK(alpha.dim() >= 1, "alpha must have a group dimension");
+        groups = alpha.size(0);
+        numel = groups * q * N;
+    } else {
+        TORCH_CHECK(kind == torch::kFloat16 || kind == torch::kInt16 || kind == torch::kInt8, "unsupported alpha dtype ", c10::toString(kind));
+        TORCH_CHECK(alpha.dim() >= 3, "block alpha must be [K/8, wbit, groups, ..]");
+        if (kind == torch::kInt8) {
+            TORCH_CHECK(alpha.dim() == 4, "int8 alpha must be [kSize/8, nb, num_groups, num_apot]");
+            per = alpha.size(3);
+        }
+        groups = alpha.size(2);
+        numel = (K / 8) * q * groups * per;
+    }
+    require(alpha, kind, "alpha");
+    TORCH_CHECK(alpha.numel() == numel, "alpha must hold ", numel, " elements, has ", alpha.numel());
+    c10::cuda::CUDAGuard guard(dev);
+    const torch::Tensor rows = x.reshape({-1, K}).to(torch::kFloat16).contiguous();
+    const int64_t M = rows.size(0);
+    auto shape = x.sizes().vec();
+    shape.back() = N;
+    torch::Tensor out = torch::empty(shape, rows.options().requires_grad(false));
+    torch::Tensor b16;
+    if (bias.has_value()) {
+        b16 = bias->detach();
+        if (b16.scalar_type() != torch::kFloat16 || !b16.is_contiguous()) b16 = b16.to(torch::kFloat16).contiguous();
+        TORCH_CHECK(b16.numel() == N && b16.device() == dev, "bias must hold ", N, " elements on the input's device");
+    }
+    void *stream = at::cuda::getCurrentCUDAStream(dev.index()).stream();
+    const void *bw = bWeight.data_ptr(), *al = alpha.data_ptr(), *bp = b16.defined() ? b16.data_ptr() : nullptr;
+    const char *xp = static_cast<const char *>(rows.data_ptr());
+    char *yp = static_cast<char *>(out.data_ptr());
+    const int layout = kind == torch::kInt8 ? -1 : (kind == torch::kInt16 ? 2 : (row_layout ? 0 : 1));
+    bool many = layout >= 0 && M > SAL_MAX_M;
+    for (int64_t r0 = 0; r0 < M;) {
+        const int m = (int)std::min<int64_t>(M - r0, many ? SAL_MAX_ROWS : SAL_MAX_M);
+        const size_t need = many ? sal_lutgemm_rows_workspace_bytes(m) : sal_workspace_bytes(m, (int)N);
+        const torch::Tensor ws = g_scratch.get(dev.index(), stream, need);
+        const void *xr = xp + (size_t)r0 * K * 2;
+        void *yr = yp + (size_t)r0 * N * 2;
+        int rc;
+        if (many) {
+            rc = sal_lutgemm_rows(layout, bw, al, bp, xr, yr, m, (int)K, (int)N, (int)q, (int)groups, 0, ws.data_ptr(), (size_t)ws.numel(), stream);
+            if (rc == SAL_E_UNSUPPORTED || rc == SAL_E_SHAPE) {   // a shape the tensor-core product does not take (or not at all, as the next call tells)
+                many = false;
+                continue;
+            }
+        } else if (layout == 0) {
+            rc = sal_lutgemv_shift_scale(bw, al, bp, xr, yr, m, (int)K, (int)N, (int)q, (int)groups, 0, ws.data_ptr(), (size_t)ws.numel(), stream);
+        } else if (layout == 1) {
+            rc = sal_lutgemm_block(bw, al, bp, xr, yr, m, (int)K, (int)N, (int)q, (int)groups, 0, ws.data_ptr(), (size_t)ws.numel(), stream);
+        } else if (layout == 2) {
+            rc = sal_lutgemm_block_shift(bw, al, bp, xr, yr, m, (int)K, (int)N, (int)q, (int)groups, 0, ws.data_ptr(), (size_t)ws.numel(), stream);
+        } else {
+            rc = sal_lutgemm_block_shift_int8(bw, al, bp, xr, yr, m, (int)K, (int)N, (int)q, (int)groups, (int)per, 0, ws.data_ptr(), (size_t)ws.numel(),
+                                              stream);
+        }
+        check_status(rc, "LutLinear");
+        r0 += m;
+    }
+    return out.to(x.scalar_type());
+}
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
@@ -177,5 +255,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("lutgemv_fused", &lutgemv_fused, "output = bias + product (mode A), optionally with programmatic dependent launch",
           py::arg("output"), py::arg("bWeight"), py::arg("alpha"), py::arg("bias"), py::arg("d_input"), py::arg("mSize"), py::arg("kSize"),
           py::arg("nb"), py::arg("num_groups"), py::arg("pdl") = false, release());
+    m.def("lut_linear", &lut_linear, "the product of LutLinear.forward: rows of x times the packed layer, bias added", py::arg("x"), py::arg("bWeight"),
+          py::arg("alpha"), py::arg("bias"), py::arg("K"), py::arg("N"), py::arg("wbit"), py::arg("row_layout"), release());
     m.def("sal_version", []() { return sal_version(); });
 }

@@ -18,6 +18,7 @@ and the bias add is fused into the kernel.
 from __future__ import annotations
 
 import math
+import os
 
 import torch
 import torch.nn as nn
@@ -25,6 +26,20 @@ import torch.nn as nn
 from . import lutgemm
 
 APOT_NONE = -128
+
+_native = None   # the compiled module's lut_linear; False where the module has not been built
+
+
+def _native_linear():
+    """``lut_linear`` of the compiled module (csrc/lutgemm_ext.cpp), or False: then `forward` takes the steps in Python."""
+    global _native
+    if _native is None:
+        from . import build
+
+        _lib = lutgemm._lib
+        _lib.load()   # the module links to the library by name: the one loaded here (SAL_LUTGEMM_LIBRARY) is the one it finds
+        _native = getattr(lutgemm.compiled_module(), "lut_linear", False) if os.path.exists(build.extension_path()) else False
+    return _native
 
 
 class LutLinear(nn.Module):
@@ -84,6 +99,9 @@ class LutLinear(nn.Module):
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         if x.shape[-1] != self.K:
             raise RuntimeError(f"last dim of the input must be {self.K}, got {x.shape[-1]}")
+        native = _native if _native is not None else _native_linear()
+        if native and x.is_cuda:
+            return native(x, self.binaryWeight, self.alpha, self.bias, self.K, self.N, self.wbit, self.alpha_layout == "row")
         out_shape = list(x.shape[:-1]) + [self.N]
         dtype = x.dtype
         x2 = x.reshape(-1, self.K).to(torch.float16).contiguous()
