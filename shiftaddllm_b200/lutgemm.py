@@ -243,7 +243,9 @@ class GroupedLaunch:
 
 class LaunchSequence:
     """Several prepared launches enqueued by one call into the library (`sal_launch_prepared_sequence`): what a
-    decoder block or a whole token is.  All launches must belong to one device."""
+    decoder block or a whole token is.  All launches must belong to one device.  Where no launch reads what
+    another one of the sequence writes, a launch starts to compute while the one in front of it finishes
+    (`sal_launch_prepared_sequence_overlapped`)."""
 
     def __init__(self, launches):
         self._launches = list(launches)
@@ -255,6 +257,7 @@ class LaunchSequence:
             raise RuntimeError("all launches of a sequence must be on one device")
         self._handles = (_lib._vp * len(self._launches))(*[l._handle for l in self._launches])
         self._need = max(l._need for l in self._launches)
+        self._overlap = bool(self._lib.sal_sequence_independent(self._handles, len(self._launches)))
 
     def __call__(self):
         dev = self._device
@@ -265,7 +268,10 @@ class LaunchSequence:
         ws = _workspaces.get((dev.index, stream))
         if ws is None or ws.numel() < self._need:
             ws = workspace_bytes(dev, self._need)
-        rc = self._lib.sal_launch_prepared_sequence(self._handles, len(self._launches), None, ws.data_ptr(), ws.numel(), stream)
+        if self._overlap:
+            rc = self._lib.sal_launch_prepared_sequence_overlapped(self._handles, len(self._launches), ws.data_ptr(), ws.numel(), stream)
+        else:
+            rc = self._lib.sal_launch_prepared_sequence(self._handles, len(self._launches), None, ws.data_ptr(), ws.numel(), stream)
         if rc != 0:
             _lib.check(rc, "sal_launch_prepared_sequence")
 
