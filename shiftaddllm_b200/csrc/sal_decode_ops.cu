@@ -562,7 +562,7 @@ __device__ __forceinline__ float rope_in(const void *p, size_t i) {
 // barrier, CTA 0 of the cluster reads all of them and writes the output, a second barrier keeps the others (and their
 // shared memory) alive until it has.  Replaces partials -> fence -> counter -> re-read through L2; no scratch is used.
 template <int G, bool STAGE_V, int ROPE, bool CLUSTER = false>
-__global__ void __launch_bounds__(ATTN_WARPS * 32) attention_split_kernel(const void *q, __half *k_cache, __half *v_cache,
+__global__ void __launch_bounds__(ATTN_WARPS * 32, (!STAGE_V && G == 1) ? 4 : 1) attention_split_kernel(const void *q, __half *k_cache, __half *v_cache,
                                                                           const int64_t *pos_p, __half *out, float *partial,
                                                                           unsigned *counters, int kv_heads, int hd,
                                                                           int max_len, float scale, int nsplit,
@@ -583,7 +583,10 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32) attention_split_kernel(const 
     __shared__ float s_w[ATTN_MAX_SPLIT][G];
     __shared__ int s_is_last;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    constexpr int NW = ATTN_WARPS, U = 4;
+    // Row reads in flight per lane.  Staged rows are in shared memory already.  Rows read from global memory (sequences in lock step: one
+    // slice per kv head and sequence, 134 MB a launch for 16 x 32 heads at 512 positions) are what bounds the kernel: eight per lane, with
+    // four CTAs per SM (50.6 -> 42.3 us a launch there, 46 -> 64 registers).  More query heads per kv head leave no registers for that.
+    constexpr int NW = ATTN_WARPS, U = (!STAGE_V && G == 1) ? 8 : 4;
     float *qf = smem_f;                  // [G][hd], pre-scaled
     float *sc = qf + G * hd;             // [G][slice_cap]
     float *obuf = sc + G * slice_cap;    // [NW][G][hd]
