@@ -297,11 +297,23 @@ __global__ void __launch_bounds__(THREADS, 1) bcq_mma_kernel(const __grid_consta
                     __syncwarp();
                 } else {
                     const int words = pr.K / 32;
-#pragma unroll 1
+                    const bool pairs = (pr.N & 1) == 0 && (reinterpret_cast<uintptr_t>(pr.bw) & 7) == 0;
+#pragma unroll 2
                     for (int r = 0; r < UNIT_WORDS * Q; ++r) {
                         const int kk = k * UNIT_WORDS + r / Q;
                         const bool row_ok = kk < words;
                         const uint32_t *src = pr.bw + ((size_t)(row_ok ? kk : 0) * Q + r % Q) * pr.N;
+                        if (pairs) {
+#pragma unroll
+                            for (int c = 0; c < TILE_N; c += 64) {
+                                const int n = sg.n0 + c + 2 * lane;
+                                const bool ok = row_ok && n < pr.N;
+                                asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst + (uint32_t)(r * TILE_N + c + 2 * lane) * 4),
+                                             "l"(src + (ok ? n : 0)), "r"(ok ? 8 : 0)
+                                             : "memory");
+                            }
+                            continue;
+                        }
 #pragma unroll
                         for (int c = 0; c < TILE_N; c += 32) {
                             const int n = sg.n0 + c + lane;
@@ -698,8 +710,24 @@ int build(const sal_problem *problems, int count, AlphaLayout layout, unsigned f
     P.total_units = units;
     // CTAs: one per SM, as far as there are units and the scratch buffer holds their partial sums (two slots of mt x 128
     // floats each); without scratch, one per output tile
+    // Where whole numbers of shares per tile fill most of the SMs, runs are cut at tile borders (run_begin does so by itself): every
+    // CTA has one segment instead of two, and a tile fewer shares to sum, which for many rows costs as much as the product.  At least
+    // four units per share, or eight shares.  us with 148 CTAs / with whole shares, for 64 and 256 rows: 4096 x 4096, 3 planes 20.3 / 17.3
+    // and 43.3 / 36.2 (128 CTAs), 4096 x 1024 15.3 / 13.5 and 45.4 / 32.3 (64), 2048 x 2048 14.8 / 11.2 and 37.7 / 29.2 (128), 8192 x 8192,
+    // 2 planes 32.7 / 32.0 and 70.2 / 73.1 (128); with 86 of 148 (4096 x 11008) 36.7 / 45.8, hence the line at 86 %.
+    // Not where rows are copied by plain instructions: a unit takes three times as long there (2080 x 1378, 3 rows: 18.4 / 20.5).
     const size_t slot_bytes = (size_t)2 * P.mt * TILE_N * sizeof(float);
     long long ctas = sms < units ? sms : units;
+    bool same_k = true;
+    for (int i = 1; i < count; ++i) same_k = same_k && P.p[i].ku == P.p[0].ku;
+    if (same_k && tma_scales && tiles <= sms) {
+        const int ku = P.p[0].ku, most = ku / 4 > 8 ? ku / 4 : 8;
+        int shares = sms / tiles;
+        const bool enough = shares > most;
+        if (shares > most) shares = most;
+        if (shares > ku) shares = ku;
+        if (enough || shares * tiles * 100 >= 86 * sms) ctas = (long long)shares * tiles;
+    }
     if (ws_bytes < WS_PARTIALS + b.act_bytes) {
         if (b.act_bytes) return SAL_E_WORKSPACE;
         ctas = 0;
