@@ -245,9 +245,9 @@ class LaunchSequence:
     """Several prepared launches enqueued by one call into the library (`sal_launch_prepared_sequence`): what a
     decoder block or a whole token is.  All launches must belong to one device.  Where no launch reads what
     another one of the sequence writes, a launch starts to compute while the one in front of it finishes
-    (`sal_launch_prepared_sequence_overlapped`)."""
+    (`sal_launch_prepared_sequence_overlapped`); ``overlap=False``: each one waits for the one in front at its start."""
 
-    def __init__(self, launches):
+    def __init__(self, launches, overlap: bool = True):
         self._launches = list(launches)
         if not self._launches:
             raise RuntimeError("an empty launch sequence")
@@ -257,7 +257,7 @@ class LaunchSequence:
             raise RuntimeError("all launches of a sequence must be on one device")
         self._handles = (_lib._vp * len(self._launches))(*[l._handle for l in self._launches])
         self._need = max(l._need for l in self._launches)
-        self._overlap = bool(self._lib.sal_sequence_independent(self._handles, len(self._launches)))
+        self._overlap = overlap and bool(self._lib.sal_sequence_independent(self._handles, len(self._launches)))
 
     def __call__(self):
         dev = self._device
