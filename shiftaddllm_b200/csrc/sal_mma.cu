@@ -30,9 +30,10 @@
 // contiguous runs.  A tile that several CTAs share is summed by the last of them to arrive, in ascending order of K
 // (deterministic), from fp32 partial sums in the scratch buffer.
 //
-// What bounds it: up to 64 rows the operand warps' chain per unit (wait for the ring, 32 logic operations per word and plane, tensor-memory
-// store, its completion, two barriers), 0.66 / 0.9 / 1.1 us a unit for 2 / 3 / 4 planes against 0.13 to 0.26 us that the planes take to
-// arrive; at 256 rows the tensor core (12 instructions of 128 clocks per plane and 384 features).  Measured in us, before (tables, a pass
+// What bounds it: a unit takes 0.66 / 0.9 / 1.1 us for 2 / 3 / 4 planes up to 64 rows, against 0.13 to 0.26 us that its planes take to
+// arrive.  About half of that the MMA warp waits for activations and the operand warps for the stages it frees; the operands
+// themselves (32 logic operations per word and plane, tensor-memory stores) are some 900 clocks.  At 256 rows the tensor core (128
+// clocks per instruction, 8 per plane and unit) and the same wait.  Measured in us, before (tables, a pass
 // per pair of rows or per row) and here: 4096 x 11008, 4 planes, 8 rows 31 -> 27, 64 rows 174 -> 36; 11008 x 4096, 3 planes, 16 rows
 // 42 -> 25; 28672 x 8192, 2 planes, 64 rows 540 -> 82; block layout, 11008 x 4096, 3 planes, 128 rows 959 -> 49.  Steps on the way: the
 // scales by TMA instead of by plain loads in the staging warps; sixteen operand warps instead of eight; the activations by TMA and
