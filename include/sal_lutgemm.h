@@ -264,8 +264,9 @@ int sal_launch_prepared_sequence(const sal_prepared *const *prepared, int count,
                                  size_t workspace_bytes, void *stream);
 /* The same for launches none of which reads (x, x_mul) what another one of them writes (y): a launch then computes while
  * the one in front of it finishes and waits for it only before it writes.  Operands may come from whatever the stream ran before the
- * sequence.  sal_sequence_independent tells (1 / 0) whether that holds for the memory the launches were prepared with, all of them
- * were prepared with SAL_PDL and run on the one-row kernel without exchange. */
+ * sequence: the first launch is an ordinary one (no programmatic launch), which starts when all of that has finished.
+ * sal_sequence_independent tells (1 / 0) whether that holds for the memory the launches were prepared with, all of them
+ * were prepared with SAL_PDL and run on the table kernel without exchange. */
 int sal_sequence_independent(const sal_prepared *const *prepared, int count);
 int sal_launch_prepared_sequence_overlapped(const sal_prepared *const *prepared, int count, void *workspace, size_t workspace_bytes,
                                             void *stream);

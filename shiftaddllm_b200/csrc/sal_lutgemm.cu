@@ -114,19 +114,22 @@ struct TileParams {
     int accumulate;
     int ablate;  // measurement builds (-DSAL_MEASURE) only: bit0 skip alpha loads, bit1 skip table builds, bit2 skip
                  // lookups; block mode: bit3 skip the multiplier decode + stores, bit4 skip the per-tile barrier
-    int dependence;   // of this launch on the launches in front of it, see Dependence
+    int wait_last;    // see Dependence
     int *status;
     ExchangeParams ex;
 };
 
-// Launches of a sequence whose operands no launch of the sequence writes need not wait for one another before they start
-// to compute, only before they write (scratch and outputs).  A launch that merely waits at its start leaves every SM idle from
-// the end of its last CTA of the launch in front to the end of that launch's last CTA anywhere: about 4 of the 21 us of a
-// LLaMA-2-7B block launch.
+// How a launch depends on the launch in front of it.  A launch that merely waits at its start leaves every SM idle from the end of
+// its last CTA of the launch in front to the end of that launch's last CTA anywhere: about 4 of the 21 us of a LLaMA-2-7B block launch.
+// Launches of a sequence whose operands no launch of the sequence writes need not do so: they compute first and wait only before they
+// write (scratch and outputs).  griddepcontrol.wait makes visible what the launch in front wrote, and only to the grid that waits; what is
+// read ahead of it must have been complete before the grid could start at all.  So the first launch of such a sequence is an ordinary one
+// (no programmatic launch attribute): the stream starts it only when all earlier work has finished and its writes are visible, and
+// every later launch of the sequence starts after it has started.
 enum Dependence {
-    WAIT_FIRST = 0,   // operands may come from the launch in front
-    SEQUENCE_HEAD,    // the same, and the next launch may start only once this one has waited: it does not wait itself
-    WAIT_LAST         // operands are older than the sequence: wait in front of the epilogue
+    WAIT_FIRST,      // operands may come from the launch in front
+    SEQUENCE_HEAD,   // ordinary launch: starts when all earlier work of the stream has finished
+    WAIT_LAST        // operands are older than the sequence's head: wait in front of the epilogue
 };
 
 // Parts of the kernel can be switched off to time the others; only in measurement builds, so that
@@ -487,7 +490,7 @@ __global__ void __launch_bounds__(TileCfg<Q, NCW>::THREADS, (NCW <= 8 ? 2 : 1))
         fence_barrier_init();
     }
     __syncthreads();
-    if (P.dependence != SEQUENCE_HEAD) pdl_launch_dependents();
+    pdl_launch_dependents();
 
     if (warp == NCW) {
         // ------------------------------ producer warp ------------------------------
@@ -754,10 +757,7 @@ __global__ void __launch_bounds__(TileCfg<Q, NCW>::THREADS, (NCW <= 8 ? 2 : 1))
     uint32_t mbuf = 0;  // byte offset of the multiplier buffer the current tile uses (two buffers, alternating)
 
     [[maybe_unused]] const long long t_wait0 = SAL_CYCLES();
-    if (P.dependence != WAIT_LAST) {
-        pdl_wait();  // activations, bias, y and the scratch buffer may be written by the previous kernel
-        if (P.dependence == SEQUENCE_HEAD) pdl_launch_dependents();
-    }
+    if (!P.wait_last) pdl_wait();  // activations, bias, y and the scratch buffer may be written by the previous kernel
     [[maybe_unused]] const long long t_wait1 = SAL_CYCLES();
     [[maybe_unused]] long long t_data = 0, t_build = 0;
 
@@ -987,7 +987,7 @@ __global__ void __launch_bounds__(TileCfg<Q, NCW>::THREADS, (NCW <= 8 ? 2 : 1))
     }
 
     // ---------------------------------- epilogue ----------------------------------
-    if (P.dependence == WAIT_LAST) pdl_wait();
+    if (P.wait_last) pdl_wait();
 #ifdef SAL_MEASURE
     if (lane == 0 && (warp == 0 || warp == NCW - 1) && blockIdx.x < 512 && blockIdx.y == 0) {
         unsigned long long *d = g_cta_timers + (size_t)(blockIdx.x * 2 + (warp ? 1 : 0)) * 8;
@@ -1758,7 +1758,8 @@ int launch_built(const BuiltLaunch &L, void *workspace, size_t ws_bytes, int slo
     if (L.ws_need > 0 && (workspace == nullptr || ws_bytes < L.ws_need)) return SAL_E_WORKSPACE;
     TileParams P = L.P;
     P.status = workspace ? reinterpret_cast<int *>(workspace) : nullptr;
-    P.dependence = dependence;
+    P.wait_last = dependence == WAIT_LAST;
+    const unsigned flags = dependence == SEQUENCE_HEAD ? L.flags & ~SAL_PDL : L.flags;
     if (slot >= 0) P.ex.slot = slot;
     for (int i = 0; i < P.count; ++i) {
         if (L.counter_off[i] < 0) continue;
@@ -1783,10 +1784,10 @@ int launch_built(const BuiltLaunch &L, void *workspace, size_t ws_bytes, int slo
     const bool abs_ok = dev->smem_base == (int)SMEM_DYNAMIC_BASE;
     cudaError_t e;
     switch (L.q) {
-        case 1: e = launch_tiled<1>(P, L.ctas, L.rows, L.row_groups, L.swiglu, L.atomic_out, L.smem, L.flags, abs_ok, stream); break;
-        case 2: e = launch_tiled<2>(P, L.ctas, L.rows, L.row_groups, L.swiglu, L.atomic_out, L.smem, L.flags, abs_ok, stream); break;
-        case 3: e = launch_tiled<3>(P, L.ctas, L.rows, L.row_groups, L.swiglu, L.atomic_out, L.smem, L.flags, abs_ok, stream); break;
-        default: e = launch_tiled<4>(P, L.ctas, L.rows, L.row_groups, L.swiglu, L.atomic_out, L.smem, L.flags, abs_ok, stream); break;
+        case 1: e = launch_tiled<1>(P, L.ctas, L.rows, L.row_groups, L.swiglu, L.atomic_out, L.smem, flags, abs_ok, stream); break;
+        case 2: e = launch_tiled<2>(P, L.ctas, L.rows, L.row_groups, L.swiglu, L.atomic_out, L.smem, flags, abs_ok, stream); break;
+        case 3: e = launch_tiled<3>(P, L.ctas, L.rows, L.row_groups, L.swiglu, L.atomic_out, L.smem, flags, abs_ok, stream); break;
+        default: e = launch_tiled<4>(P, L.ctas, L.rows, L.row_groups, L.swiglu, L.atomic_out, L.smem, flags, abs_ok, stream); break;
     }
     return cuda_ok(e) ? SAL_OK : SAL_E_LAUNCH;
 }
