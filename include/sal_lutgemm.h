@@ -89,7 +89,7 @@ int sal_device_ok(void);
  * Scratch ("workspace") for the deterministic split-K reduction.  The caller
  * allocates `sal_workspace_bytes(M, N)` bytes of device memory once, zero-fills
  * it once (cudaMemset), and may reuse it for any later call whose M and N are
- * not larger.  Calls sharing one workspace must be ordered on one stream.
+ * not larger.  Calls sharing one workspace must be ordered on one stream; several host threads may enqueue them.
  * For a grouped launch pass the sum of N over the group.
  */
 size_t sal_workspace_bytes(int M, int N);

@@ -37,6 +37,7 @@
 #include <cuda_fp16.h>
 #include <mutex>
 #include <new>
+#include <shared_mutex>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -1600,6 +1601,7 @@ int run_generic(int kind, GenericParams p, void *workspace, size_t ws_bytes, cud
         }
     }
     dim3 grid((unsigned)col_blocks, (unsigned)p.M, (unsigned)p.ksplit);
+    std::shared_lock<std::shared_mutex> order(sal_scratch_order(workspace));
     switch (kind) {
         case A_ROW_F16: lutgemv_generic_kernel<A_ROW_F16><<<grid, 128, 0, stream>>>(p); break;
         case A_ROW_HALVING: lutgemv_generic_kernel<A_ROW_HALVING><<<grid, 128, 0, stream>>>(p); break;
@@ -1782,6 +1784,7 @@ int launch_built(const BuiltLaunch &L, void *workspace, size_t ws_bytes, int slo
         }
     }
     const bool abs_ok = dev->smem_base == (int)SMEM_DYNAMIC_BASE;
+    std::shared_lock<std::shared_mutex> order(sal_scratch_order(workspace));
     cudaError_t e;
     switch (L.q) {
         case 1: e = launch_tiled<1>(P, L.ctas, L.rows, L.row_groups, L.swiglu, L.atomic_out, L.smem, flags, abs_ok, stream); break;
@@ -1880,6 +1883,11 @@ int validate_grouped(const sal_problem *problems, int count, unsigned flags, boo
 }
 
 }  // namespace
+
+std::shared_mutex &sal_scratch_order(const void *workspace) {
+    static std::shared_mutex locks[64];
+    return locks[(reinterpret_cast<uintptr_t>(workspace) >> 12) % 64];   // two buffers may meet in one: they then only wait for each other
+}
 
 static int tensor_map_encoder() {
     if (g_encode_tiled) return SAL_OK;

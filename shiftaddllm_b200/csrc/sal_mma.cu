@@ -46,6 +46,8 @@
 #include <cuda_fp16.h>
 #include <stdint.h>
 
+#include <mutex>
+
 #include "sal_decode_ops.h"
 #include "sal_mma.h"
 
@@ -761,6 +763,11 @@ size_t scratch_bytes(const Built &b) {
 int launch(const Built &b, void *workspace, size_t ws_bytes, cudaStream_t stream) {
     const size_t need = scratch_bytes(b);
     if (need > 0 && (!workspace || ws_bytes < need)) return SAL_E_WORKSPACE;
+    std::shared_mutex &order = sal_scratch_order(workspace);
+    std::unique_lock<std::shared_mutex> alone(order, std::defer_lock);
+    std::shared_lock<std::shared_mutex> shared(order, std::defer_lock);
+    if (b.act_bytes) alone.lock();
+    else shared.lock();
     Params P = b.P;
     char *base = reinterpret_cast<char *>(workspace);
     P.status = reinterpret_cast<int *>(workspace);

@@ -6,6 +6,8 @@
 #include <cuda_runtime.h>
 #include <stddef.h>
 
+#include <shared_mutex>
+
 #include "sal_lutgemm.h"
 
 namespace sal_mma {
@@ -75,6 +77,11 @@ size_t scratch_bytes(const Built &b);   // 0: none
 int launch(const Built &b, void *workspace, size_t ws_bytes, cudaStream_t stream);
 
 }  // namespace sal_mma
+
+// Host threads that share a stream and with it a scratch buffer may enqueue at the same time.  A product that is one launch holds this
+// lock shared; one that passes data from launch to launch through the scratch buffer (silu(x) * x_mul of several rows) holds it alone, so
+// that no other launch on the same buffer gets in between.  Defined in sal_lutgemm.cu.
+std::shared_mutex &sal_scratch_order(const void *workspace);
 
 // Encodes the tensor map of packed planes with the given box (planes x words); defined in sal_lutgemm.cu.
 int sal_encode_planes(CUtensorMap *out, const void *bw, int K, int N, int q, int box_cols, int box_planes, int box_words);
