@@ -14,7 +14,7 @@ PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 REPO_DIR = os.path.dirname(PKG_DIR)
 SRCS = [os.path.join(PKG_DIR, "csrc", name) for name in ("sal_lutgemm.cu", "sal_mma.cu", "sal_decode_ops.cu", "sal_pack.cu")]
 HDRS = [os.path.join(REPO_DIR, "include", name) for name in ("sal_lutgemm.h", "sal_decode_ops.h", "sal_pack.h")]
-HDRS.append(os.path.join(PKG_DIR, "csrc", "sal_mma.h"))
+HDRS += [os.path.join(PKG_DIR, "csrc", name) for name in ("sal_launch.h", "sal_mma.h")]
 LIB = os.path.join(PKG_DIR, "libsal_lutgemm.so")
 
 NVCC_FLAGS = [

@@ -6,6 +6,7 @@
 #include <stdint.h>
 
 #include "sal_decode_ops.h"
+#include "sal_launch.h"
 #include "sal_lutgemm.h"
 
 namespace {
@@ -925,16 +926,8 @@ int launch_attention_variant(size_t smem, const void *q, const void *k_cache, co
                              int kv_heads, int hd, int max_len, float scale, void *workspace, int nsplit, int slice_cap,
                              const RopeArgs &ra, cudaStream_t stream, int batch = 1, const SeqStrides &ss = SeqStrides{}) {
     if (smem + 2048 > 48 * 1024) {   // the kernel's static shared memory counts against the default limit too
-        // the attribute belongs to the (function, device) pair: remember it per device ordinal
-        static size_t configured[64];
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return SAL_E_DEVICE;
-        if (configured[dev] < smem) {
-            if (cudaFuncSetAttribute(attention_split_kernel<G, STAGE_V, ROPE, CLUSTER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem) != cudaSuccess)
-                return SAL_E_LAUNCH;
-            configured[dev] = smem;
-        }
+        static std::atomic<bool> configured[64];
+        if (sal_allow_shared_memory(attention_split_kernel<G, STAGE_V, ROPE, CLUSTER>, configured) != cudaSuccess) return SAL_E_LAUNCH;
     }
     if (CLUSTER) {   // the slices of a kv head are one thread-block cluster (at most 8: the portable size)
         cudaLaunchConfig_t cfg = {};

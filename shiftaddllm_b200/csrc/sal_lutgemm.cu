@@ -42,9 +42,11 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <atomic>
 #include <type_traits>
 #include <vector>
 
+#include "sal_launch.h"
 #include "sal_lutgemm.h"
 #include "sal_mma.h"
 
@@ -1509,14 +1511,9 @@ int encode_weight_map(CUtensorMap *out, const void *bw, int K, int N, int q) {
 template <int Q, int NCW, bool ABS, int ROWS, int SWIGLU, bool EXCH = false, bool ATOMIC = false, bool BLK = false>
 cudaError_t launch_tiled_variant(const TileParams &P, int ctas, int row_groups, int smem, unsigned flags, cudaStream_t stream) {
     auto kern = lutgemv_tiled_kernel<Q, NCW, ABS, ROWS, SWIGLU, EXCH, ATOMIC, BLK>;
-    static int configured[64];
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (configured[dev] < smem) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) return e;
-        configured[dev] = smem;
-    }
+    static std::atomic<bool> configured[64];
+    const cudaError_t e = sal_allow_shared_memory(kern, configured);
+    if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)ctas, (unsigned)row_groups);
     cfg.blockDim = dim3(TileCfg<Q, NCW>::THREADS);

@@ -46,9 +46,11 @@
 #include <cuda_fp16.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <mutex>
 
 #include "sal_decode_ops.h"
+#include "sal_launch.h"
 #include "sal_mma.h"
 
 namespace sal_mma {
@@ -598,14 +600,9 @@ __global__ void __launch_bounds__(THREADS, 1) bcq_mma_kernel(const __grid_consta
 
 template <int Q>
 cudaError_t launch_q(const Built &b, const Params &P, cudaStream_t stream) {
-    static int configured[64];
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (configured[dev] < b.smem) {
-        const cudaError_t e = cudaFuncSetAttribute(bcq_mma_kernel<Q>, cudaFuncAttributeMaxDynamicSharedMemorySize, b.smem);
-        if (e != cudaSuccess) return e;
-        configured[dev] = b.smem;
-    }
+    static std::atomic<bool> configured[64];
+    const cudaError_t e = sal_allow_shared_memory(bcq_mma_kernel<Q>, configured);
+    if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)b.ctas);
     cfg.blockDim = dim3(THREADS);

@@ -61,3 +61,21 @@ def test_swiglu_rows_and_split_products_from_two_threads():
         _run(work)
         for t, ps in enumerate(problems):
             assert all(torch.equal(p["output"], a) for p, a in zip(ps, alone[t])), (rep, t)
+
+
+def test_launches_of_different_shared_memory_from_several_threads():
+    """Products whose plans ask the same kernel for different amounts of shared memory (rows, small groups, plain copies): every launch goes
+    through, whichever thread was there first."""
+    shapes = [(512, 256, 300, 128), (512, 264, 7, 128), (512, 512, 130, 128), (512, 128, 17, 128)]
+    work, problems = [], []
+    for t in range(4):
+        ps = [_problem(*shapes[(i + t) % 4][:3], 1, 10 * t + i) for i in range(8)]
+        problems += ps
+        work.append(200 * [lutgemm.prepare_grouped([p], many_rows=True) for p in ps])
+    for launches in work:
+        for launch in launches[:8]:
+            launch()
+    torch.cuda.synchronize()
+    alone = [p["output"].clone() for p in problems]
+    _run(work)
+    assert all(torch.equal(p["output"], a) for p, a in zip(problems, alone))
