@@ -609,7 +609,7 @@ cudaError_t launch_q(const Built &b, const Params &P, cudaStream_t stream) {
     cfg.dynamicSmemBytes = (size_t)b.smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
-    if ((b.flags & SAL_PDL) || b.act_bytes) {
+    if (b.flags & SAL_PDL) {
         attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;

@@ -116,7 +116,7 @@ def test_later_launches_see_what_the_stream_wrote_before_the_sequence(rows, form
         assert all(torch.equal(a, b) for a, b in zip(got, outs)), rep
 
 
-def _graph(fn):
+def graph_of(fn):
     """Kernel launches, dependencies and programmatic dependencies of what `fn` enqueues, from a graph captured of it."""
     rt = ctypes.CDLL("libcudart.so.12")
     stream, graph, nodes, edges = torch.cuda.Stream(), ctypes.c_void_p(), ctypes.c_size_t(), ctypes.c_size_t()
@@ -145,5 +145,5 @@ def test_head_of_a_sequence_is_an_ordinary_launch():
         front()
         seq()
 
-    assert _graph(both) == (4, 3, 2)
-    assert _graph(lambda: (front(), front())) == (2, 1, 1)
+    assert graph_of(both) == (4, 3, 2)
+    assert graph_of(lambda: (front(), front())) == (2, 1, 1)

@@ -10,6 +10,7 @@ import torch
 
 from shiftaddllm_b200 import _lib, lutgemm
 from shiftaddllm_b200.quant import LutLinear
+from test_gpu_sequence import graph_of
 
 pytestmark = pytest.mark.gpu
 
@@ -118,3 +119,12 @@ def test_grouped_rows_with_swiglu(m):
     ref, bound = _reference(bits, mult, act, bias)
     # silu is rounded to fp16 before the product here and in torch; a last-bit difference of its exponential moves an activation by 2**-10
     assert ((p["output"].double() - ref).abs() <= bound + 2.0 ** -10 * (act.double().abs() @ mult.sum(1).repeat_interleave(128, 0))).all()
+
+
+@pytest.mark.parametrize("pdl", [False, True])
+def test_programmatic_launch_only_where_it_was_asked_for(pdl):
+    """The two launches of a SwiGLU product: the second one may read planes and scales ahead of its dependencies only with `pdl`."""
+    bits, alpha, _, x, _ = _case(0, 8, 512, 128, 3, 128)
+    p = dict(output=torch.empty(8, 128, dtype=torch.float16, device="cuda"), bWeight=bits, alpha=alpha, bias=None, d_input=x, d_input_mul=x,
+             mSize=128, kSize=512, nb=3, num_groups=4)
+    assert graph_of(lutgemm.prepare_grouped([p], pdl=pdl)) == (2, 1, int(pdl))
