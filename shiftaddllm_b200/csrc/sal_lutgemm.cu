@@ -519,8 +519,12 @@ __global__ void __launch_bounds__(TileCfg<Q, NCW>::THREADS, (NCW <= 8 ? 2 : 1))
                     __syncwarp();
                     if (++st == stages) {
                         st = 0;
-                        if (first_round) first_round = false;
-                        else phase ^= 1u;
+                        if (first_round) {
+                            // from here on the consumers have to make room, which they do behind their own dependency wait: its time
+                            // is the kernel in front's and does not count against the limit of the wait for a slot
+                            if (!P.wait_last) pdl_wait();
+                            first_round = false;
+                        } else phase ^= 1u;
                     }
                 }
             }

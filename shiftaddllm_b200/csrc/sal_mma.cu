@@ -41,8 +41,10 @@
 // elect.sync instead of `lane == 0` (34 -> 24 us at 11008 x 4096, 1 to 16 rows).  Operands through shared memory instead of tensor
 // memory gained nothing (38 us there, before the last step).
 //
-// Every wait is bounded (about a second), recorded as SAL_E_TIMEOUT in the workspace header, and not repeated: a thread
-// that gave up once runs through to its end.
+// Every wait on a barrier is bounded (about a second) and not repeated: a thread that gave up once runs through to its end.  It is recorded
+// as SAL_E_TIMEOUT in the header of the scratch buffer (a launch without one has no place for it).  The limit covers this launch's own
+// pipeline only: a warp whose progress depends on the activations executes griddepcontrol.wait, which takes as long as the kernel in front
+// does, before its first such wait.
 #include <cuda_fp16.h>
 #include <stdint.h>
 
@@ -276,12 +278,17 @@ __global__ void __launch_bounds__(THREADS, 1) bcq_mma_kernel(const __grid_consta
         // ------------------------------------------- planes and scales -------------------------------------------
         int st = 0;
         uint32_t ph = 1;   // a fresh barrier passes a wait for the phase before its first
+        bool waited = false;
         while (next_segment(P, u, u_end, sg)) {
             const Problem &pr = P.p[sg.pi];
             const int cols = min(TILE_N, pr.N - sg.n0);
             const int gfirst = P.layout == ROW ? 0 : sg.n0 / pr.gs;   // BLOCK: the tile's groups
             const int bgroups = P.layout == ROW ? 0 : min((sg.n0 + TILE_N - 1) / pr.gs, pr.ngroups - 1) - gfirst + 1;
             for (int k = sg.k0; k < sg.k1; ++k) {
+                if (!ph && !waited) {   // the ring is full: from here on the operand warps have to make room
+                    asm volatile("griddepcontrol.wait;" ::: "memory");
+                    waited = true;
+                }
                 mbar_wait(w_empty + 8 * st, ph, P.status, live);
                 const uint32_t dst = ws + st * w_stage, bar = w_full + 8 * st;
                 const uint32_t sdst = dst + C::W_BYTES;
@@ -357,6 +364,7 @@ __global__ void __launch_bounds__(THREADS, 1) bcq_mma_kernel(const __grid_consta
         // ------------------------------------------- tensor core -------------------------------------------
         // fp32 accumulators, fp16 operands, both K-major, N = mpad, M = 128
         const uint32_t idesc = (1u << 4) | ((uint32_t)(P.mpad >> 3) << 17) | ((TILE_N >> 4) << 24);
+        asm volatile("griddepcontrol.wait;" ::: "memory");
         int xst = 0, ast = 0;
         uint32_t xph = 0, aph = 0, dph = 1;
         while (next_segment(P, u, u_end, sg)) {
@@ -413,6 +421,7 @@ __global__ void __launch_bounds__(THREADS, 1) bcq_mma_kernel(const __grid_consta
         const int word = warp - OP_WARPS;
         const uint32_t c0 = (uint32_t)(word & 1) * 4, sw = (uint32_t)(lane & 7);   // 32 rows on, the swizzle is the same
         const uint32_t o0 = ((c0 + 0) ^ sw) << 4, o1 = ((c0 + 1) ^ sw) << 4, o2 = ((c0 + 2) ^ sw) << 4, o3 = ((c0 + 3) ^ sw) << 4;
+        asm volatile("griddepcontrol.wait;" ::: "memory");
         int xst = 0;
         uint32_t xph = 0;
         while (next_segment(P, u, u_end, sg)) {
@@ -478,6 +487,10 @@ __global__ void __launch_bounds__(THREADS, 1) bcq_mma_kernel(const __grid_consta
                         sa[b] = prmt(a[0], a[2], 0x5410) ^ 0x80008000u;
                         sb[b] = prmt(a[1], a[3], 0x5410) ^ 0x80008000u;
                     }
+                }
+                if (!aph && !waited) {   // the operand stages are full: from here on the tensor core has to have the activations
+                    asm volatile("griddepcontrol.wait;" ::: "memory");
+                    waited = true;
                 }
                 mbar_wait(a_empty + 8 * ast, aph, P.status, live);
                 fence_after();

@@ -128,3 +128,35 @@ def test_programmatic_launch_only_where_it_was_asked_for(pdl):
     p = dict(output=torch.empty(8, 128, dtype=torch.float16, device="cuda"), bWeight=bits, alpha=alpha, bias=None, d_input=x, d_input_mul=x,
              mSize=128, kSize=512, nb=3, num_groups=4)
     assert graph_of(lutgemm.prepare_grouped([p], pdl=pdl)) == (2, 1, int(pdl))
+
+
+@pytest.mark.parametrize("m", [16, 1])   # tensor-core and table kernel
+def test_a_long_kernel_in_front_does_not_run_the_waits_out(m):
+    """Programmatic launches start while the ones in front still run, and their waits are limited to about a second each.  Four products of one
+    CTA and some tenths of a second each in front: the time of those must not count."""
+    k, lib = 1 << 27, _lib.load()
+    long_bits = torch.zeros(k // 32, 4, 8, dtype=torch.int32, device="cuda")
+    long_alpha, long_x = torch.ones(1, 4, 8, dtype=torch.float16, device="cuda"), torch.zeros(2, k, dtype=torch.float16, device="cuda")
+    long_y = torch.empty(2, 8, dtype=torch.float16, device="cuda")
+    bits, alpha, _, x, bias = _case(0, m, 8192, 512, 3, 128)
+    ws = torch.zeros(lib.sal_lutgemm_rows_workspace_bytes(64), dtype=torch.uint8, device="cuda")
+    y = torch.empty(m, 512, dtype=torch.float16, device="cuda")
+
+    def product():
+        assert lib.sal_lutgemv_shift_scale(bits.data_ptr(), alpha.data_ptr(), bias.data_ptr(), x.data_ptr(), y.data_ptr(), m, 8192, 512, 3, 64,
+                                           _lib.SAL_PDL, ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream) == 0
+
+    product()
+    want = y.clone()
+    y.zero_()
+    begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    begin.record()
+    for _ in range(4):
+        assert lib.sal_lutgemm_rows(0, long_bits.data_ptr(), long_alpha.data_ptr(), None, long_x.data_ptr(), long_y.data_ptr(), 2, k, 8, 4, 1,
+                                    _lib.SAL_PDL, ws.data_ptr(), 256, torch.cuda.current_stream().cuda_stream) == 0
+    product()
+    end.record()
+    torch.cuda.synchronize()
+    assert begin.elapsed_time(end) > 1500   # otherwise this shows nothing
+    assert torch.equal(y, want)
+    assert lib.sal_workspace_status(ws.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
