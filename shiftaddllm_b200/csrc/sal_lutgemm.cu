@@ -506,7 +506,12 @@ __global__ void __launch_bounds__(TileCfg<Q, NCW>::THREADS, (NCW <= 8 ? 2 : 1))
                 const int n0 = (sub_begin + sub) * CW;
 #pragma unroll 1
                 for (int b = 0; b < Q; b += C::PPS) {   // one slot per PPS planes
-                    if (!first_round) mbar_wait(empty0 + 8 * st, phase, P.status);
+                    if (!first_round && !mbar_try_wait(empty0 + 8 * st, phase)) {
+                        // The consumers make room behind their own dependency wait: its time is the kernel in front's and does not
+                        // count against the limit of the wait for a slot.
+                        if (!P.wait_last) pdl_wait();
+                        mbar_wait(empty0 + 8 * st, phase, P.status);
+                    }
                     const uint32_t full = full0 + 8 * st;
                     if (lane == 0) {
                         // columns past N are zero-filled by the TMA unit and still counted
@@ -519,12 +524,8 @@ __global__ void __launch_bounds__(TileCfg<Q, NCW>::THREADS, (NCW <= 8 ? 2 : 1))
                     __syncwarp();
                     if (++st == stages) {
                         st = 0;
-                        if (first_round) {
-                            // from here on the consumers have to make room, which they do behind their own dependency wait: its time
-                            // is the kernel in front's and does not count against the limit of the wait for a slot
-                            if (!P.wait_last) pdl_wait();
-                            first_round = false;
-                        } else phase ^= 1u;
+                        if (first_round) first_round = false;
+                        else phase ^= 1u;
                     }
                 }
             }

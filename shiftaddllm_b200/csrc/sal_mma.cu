@@ -44,7 +44,8 @@
 // Every wait on a barrier is bounded (about a second) and not repeated: a thread that gave up once runs through to its end.  It is recorded
 // as SAL_E_TIMEOUT in the header of the scratch buffer (a launch without one has no place for it).  The limit covers this launch's own
 // pipeline only: a warp whose progress depends on the activations executes griddepcontrol.wait, which takes as long as the kernel in front
-// does, before its first such wait.
+// does, before its first such wait.  The warps that issue copies and matrix instructions stop copying once they gave up, and wait (once more
+// bounded) for what they have in flight before the CTA ends; in a launch that ran as it should that has long been consumed.
 #include <cuda_fp16.h>
 #include <stdint.h>
 
@@ -118,6 +119,22 @@ __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, int *
 __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, int *status, bool &live) {
     if (mbar_try_wait(bar, parity)) return;
     if (live) live = mbar_wait_slow(bar, parity, status);
+}
+// The same for a warp that runs ahead of the dependency wait: a barrier that has to be waited for may depend on the kernel in front, so
+// that kernel is waited for first.
+__device__ __forceinline__ void mbar_wait_behind(uint32_t bar, uint32_t parity, int *status, bool &live, bool &waited) {
+    if (mbar_try_wait(bar, parity)) return;
+    if (!waited) asm volatile("griddepcontrol.wait;" ::: "memory");
+    waited = true;
+    if (live) live = mbar_wait_slow(bar, parity, status);
+}
+// Waits for the last fill of every slot of a ring: `next` is the slot that would be filled next, `empty_parity` the parity its producer
+// would wait for (1 in the first round).
+__device__ __forceinline__ void land(uint32_t full, int slots, int next, uint32_t empty_parity, int *status) {
+    bool live = true;
+    // a slot in front of `next` was last filled in this round, the others in the one before (in the first round: not at all, and a
+    // fresh barrier passes a wait for the phase before its first)
+    for (int i = 0; i < slots; ++i) mbar_wait(full + 8 * i, i < next ? empty_parity ^ 1u : empty_parity, status, live);
 }
 __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t selector) {
     uint32_t d;
@@ -284,12 +301,10 @@ __global__ void __launch_bounds__(THREADS, 1) bcq_mma_kernel(const __grid_consta
             const int cols = min(TILE_N, pr.N - sg.n0);
             const int gfirst = P.layout == ROW ? 0 : sg.n0 / pr.gs;   // BLOCK: the tile's groups
             const int bgroups = P.layout == ROW ? 0 : min((sg.n0 + TILE_N - 1) / pr.gs, pr.ngroups - 1) - gfirst + 1;
-            for (int k = sg.k0; k < sg.k1; ++k) {
-                if (!ph && !waited) {   // the ring is full: from here on the operand warps have to make room
-                    asm volatile("griddepcontrol.wait;" ::: "memory");
-                    waited = true;
-                }
-                mbar_wait(w_empty + 8 * st, ph, P.status, live);
+            for (int k = sg.k0; k < sg.k1 && live; ++k) {
+                mbar_wait_behind(w_empty + 8 * st, ph, P.status, live, waited);
+                live = __all_sync(0xffffffffu, live);   // the warp stops as one
+                if (!live) break;
                 const uint32_t dst = ws + st * w_stage, bar = w_full + 8 * st;
                 const uint32_t sdst = dst + C::W_BYTES;
                 const int g0 = pr.gshift >= 0 ? (k * UNIT_WORDS) >> pr.gshift : (k * UNIT_WORDS) / pr.gw;   // ROW: first group of the unit
@@ -360,6 +375,7 @@ __global__ void __launch_bounds__(THREADS, 1) bcq_mma_kernel(const __grid_consta
             }
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
+        land(w_full, P.w_stages, st, ph, P.status);
     } else if (warp == MMA_WARP) {
         // ------------------------------------------- tensor core -------------------------------------------
         // fp32 accumulators, fp16 operands, both K-major, N = mpad, M = 128
@@ -367,6 +383,7 @@ __global__ void __launch_bounds__(THREADS, 1) bcq_mma_kernel(const __grid_consta
         asm volatile("griddepcontrol.wait;" ::: "memory");
         int xst = 0, ast = 0;
         uint32_t xph = 0, aph = 0, dph = 1;
+        bool any = false;
         while (next_segment(P, u, u_end, sg)) {
             mbar_wait(d_empty, dph, P.status, live);
             dph ^= 1u;
@@ -390,7 +407,10 @@ __global__ void __launch_bounds__(THREADS, 1) bcq_mma_kernel(const __grid_consta
                 if (++ast == P.a_stages) ast = 0, aph ^= 1u;
                 if ((step & 1) && ++xst == P.x_units) xst = 0, xph ^= 1u;
             }
+            any = true;
         }
+        bool once = true;
+        if (any) mbar_wait(d_full, dph, P.status, once);   // the last segment's commit
     } else if (warp == X_WARP) {
         // ------------------------------------------- activations: fetch -------------------------------------------
         asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -398,8 +418,10 @@ __global__ void __launch_bounds__(THREADS, 1) bcq_mma_kernel(const __grid_consta
         uint32_t xph = 1;
         while (next_segment(P, u, u_end, sg)) {
             const Problem &pr = P.p[sg.pi];
-            for (int k = sg.k0; k < sg.k1; ++k) {
+            for (int k = sg.k0; k < sg.k1 && live; ++k) {
                 mbar_wait(x_empty + 8 * xst, xph, P.status, live);
+                live = __all_sync(0xffffffffu, live);   // the warp stops as one
+                if (!live) break;
                 if (elect_one()) {   // rows past M and features past K are zero-filled and counted
                     const uint32_t bar = x_raw + 8 * xst, dst = xs + 2 * xst * x_bytes;
                     mbar_expect_tx(bar, 2 * x_bytes);
@@ -414,6 +436,7 @@ __global__ void __launch_bounds__(THREADS, 1) bcq_mma_kernel(const __grid_consta
                 if (++xst == P.x_units) xst = 0, xph ^= 1u;
             }
         }
+        land(x_raw, P.x_units, xst, xph, P.status);
     } else if (warp >= OP_WARPS) {
         // ------------------------------------------- activations: reorder -------------------------------------------
         // A warp takes one word (32 features, 64 bytes) of every row; a lane's row is read and written in place, features t and t + 16
@@ -488,11 +511,7 @@ __global__ void __launch_bounds__(THREADS, 1) bcq_mma_kernel(const __grid_consta
                         sb[b] = prmt(a[1], a[3], 0x5410) ^ 0x80008000u;
                     }
                 }
-                if (!aph && !waited) {   // the operand stages are full: from here on the tensor core has to have the activations
-                    asm volatile("griddepcontrol.wait;" ::: "memory");
-                    waited = true;
-                }
-                mbar_wait(a_empty + 8 * ast, aph, P.status, live);
+                mbar_wait_behind(a_empty + 8 * ast, aph, P.status, live, waited);
                 fence_after();
                 const uint32_t dst = tlane + d_cols + ast * C::A_COLS + (wi & 1) * 16;
 #pragma unroll
