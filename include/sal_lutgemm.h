@@ -178,7 +178,8 @@ int sal_lutgemm_block_shift_int8(const void *bw, const void *alpha_i8, const voi
  * [K/8][q][num_groups], 2: uint16 (three 3-bit exponents) of that shape, groups along N of a multiple of 16 columns.
  * x must be 16-byte aligned and q <= 4; what it does not take is SAL_E_UNSUPPORTED.  The result has the value of
  * sal_lutgemv_shift_scale / sal_lutgemm_block / sal_lutgemm_block_shift on the same rows.  With less scratch than
- * sal_lutgemm_rows_workspace_bytes(M) (zero-filled once, as above) fewer SMs share the work.
+ * sal_lutgemm_rows_workspace_bytes(M) (zero-filled once, as above) fewer SMs share the work; sal_workspace_bytes(M, N) is at least
+ * that for M > 1.  The order of summation, and so the last bit, follows from the shape if the scratch has that size, whatever more it has.
  */
 size_t sal_lutgemm_rows_workspace_bytes(int M);
 int sal_lutgemm_rows(int alpha_layout, const void *bw, const void *alpha, const void *bias, const void *x, void *y, int M, int K, int N,

@@ -1959,7 +1959,10 @@ int sal_device_ok(void) {
 size_t sal_workspace_bytes(int M, int N) {
     if (M < 1) M = 1;
     if (N < 1) N = 1;
-    return WS_PARTIAL_OFFSET + (size_t)M * (size_t)N * MAX_SPLIT * sizeof(float);
+    const size_t tables = WS_PARTIAL_OFFSET + (size_t)M * (size_t)N * MAX_SPLIT * sizeof(float);
+    // several rows may go to the tensor cores, whose split must not be cut down to the scratch buffer at hand
+    const size_t rows = M > 1 ? sal_lutgemm_rows_workspace_bytes(M) : 0;
+    return tables > rows ? tables : rows;
 }
 
 int sal_workspace_status(void *workspace, void *stream) {
@@ -2143,8 +2146,7 @@ int sal_lutgemm_block_shift_int8(const void *bw, const void *alpha_i8, const voi
 }
 
 size_t sal_lutgemm_rows_workspace_bytes(int M) {
-    const int mt = M < 1 ? 1 : (M > 256 ? 256 : M);
-    return WS_PARTIAL_OFFSET + (size_t)148 * 2 * 128 * mt * sizeof(float);
+    return sal_mma::full_scratch_bytes(M);
 }
 
 int sal_lutgemm_rows(int alpha_layout, const void *bw, const void *alpha, const void *bias, const void *x, void *y, int M, int K, int N,

@@ -73,6 +73,7 @@ constexpr int S_PITCH_ROW = 272, S_PITCH_ROW_TMA = 256, S_PITCH_BLOCK = 32, S_PI
 constexpr int TMEM_COLS = 512;
 constexpr int MAX_MT = 256;          // rows of a row tile
 constexpr size_t WS_HEADER = 256, WS_PARTIALS = 16384;
+constexpr int MAX_CTAS = 148;        // one per SM
 constexpr int MAX_COUNTERS = (int)(WS_PARTIALS - WS_HEADER) / 4;
 
 template <int Q>
@@ -659,6 +660,11 @@ bool eligible(const void *bw, const void *alpha, const void *x, int M, int K, in
     return N % num_groups == 0 && (N / num_groups) % 16 == 0;   // at most nine groups meet a tile of 128 columns
 }
 
+size_t full_scratch_bytes(int M) {
+    const int mt = M < 1 ? 1 : (M > MAX_MT ? MAX_MT : M);
+    return WS_PARTIALS + (size_t)MAX_CTAS * 2 * TILE_N * mt * sizeof(float);
+}
+
 int build(const sal_problem *problems, int count, AlphaLayout layout, unsigned flags, size_t ws_bytes, int sms, Built *out) {
     Built &b = *out;
     b = Built{};
@@ -741,7 +747,8 @@ int build(const sal_problem *problems, int count, AlphaLayout layout, unsigned f
     }
     P.total_units = units;
     // CTAs: one per SM, as far as there are units and the scratch buffer holds their partial sums (two slots of mt x 128
-    // floats each); without scratch, one per output tile
+    // floats each; the documented size holds them all, so that the split and with it the last bits follow from the shape alone);
+    // without scratch, or with so little that it would leave SMs idle, one per output tile
     // Where whole numbers of shares per tile fill most of the SMs, runs are cut at tile borders (run_begin does so by itself): every
     // CTA has one segment instead of two, and a tile fewer shares to sum, which for many rows costs as much as the product.  At least
     // four units per share, or eight shares.  us with 148 CTAs / with whole shares, for 64 and 256 rows: 4096 x 4096, 3 planes 20.3 / 17.3
@@ -749,6 +756,7 @@ int build(const sal_problem *problems, int count, AlphaLayout layout, unsigned f
     // 2 planes 32.7 / 32.0 and 70.2 / 73.1 (128); with 86 of 148 (4096 x 11008) 36.7 / 45.8, hence the line at 86 %.
     // Not where rows are copied by plain instructions: a unit takes three times as long there (2080 x 1378, 3 rows: 18.4 / 20.5).
     const size_t slot_bytes = (size_t)2 * P.mt * TILE_N * sizeof(float);
+    if (sms > MAX_CTAS) sms = MAX_CTAS;
     long long ctas = sms < units ? sms : units;
     bool same_k = true;
     for (int i = 1; i < count; ++i) same_k = same_k && P.p[i].ku == P.p[0].ku;
@@ -768,7 +776,7 @@ int build(const sal_problem *problems, int count, AlphaLayout layout, unsigned f
         if (ctas > fit) ctas = fit;
     }
     if (tiles > MAX_COUNTERS) ctas = 0;
-    P.whole_tiles = ctas < 1 || (ctas < sms && ctas < tiles && tiles <= sms);
+    P.whole_tiles = ctas < (tiles < sms ? tiles : sms);   // of what the scratch buffer leaves
     b.ctas = P.whole_tiles ? tiles : (int)ctas;
     b.ws_need = P.whole_tiles ? 0 : WS_PARTIALS + (size_t)b.ctas * slot_bytes;
     const int d_cols = (P.mpad + 31) & ~31, a_cols = 32 * b.q;

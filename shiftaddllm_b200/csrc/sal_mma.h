@@ -74,6 +74,8 @@ bool eligible(const void *bw, const void *alpha, const void *x, int M, int K, in
 // Plans one launch; `ws_bytes` of scratch will be there (0: none).  All problems share M, q and the layout.
 int build(const sal_problem *problems, int count, AlphaLayout layout, unsigned flags, size_t ws_bytes, int sms, Built *out);
 size_t scratch_bytes(const Built &b);   // 0: none
+// Scratch with which the split of a product of M rows (without x_mul) follows from its shape alone
+size_t full_scratch_bytes(int M);
 int launch(const Built &b, void *workspace, size_t ws_bytes, cudaStream_t stream);
 
 }  // namespace sal_mma

@@ -120,3 +120,12 @@ def test_planner_invariants_over_many_shapes(lib):
                     assert info.stages >= (2 if q == 4 else 1)
                     assert info.smem_bytes <= 115712
     assert seen_tiled > 500
+
+
+def test_scratch_of_several_rows_holds_every_split():
+    """What a caller is told to allocate for a small-batch product is what the tensor-core product needs for its full split, whatever N."""
+    lib = _lib.load()
+    for m in (2, 7, 16, 64):
+        for n in (8, 130, 592, 4096):
+            assert lib.sal_workspace_bytes(m, n) >= max(lib.sal_lutgemm_rows_workspace_bytes(m), 16384 + m * n * 64 * 4)
+    assert lib.sal_lutgemm_rows_workspace_bytes(64) == 16384 + 148 * 2 * 128 * 64 * 4

@@ -160,3 +160,37 @@ def test_a_long_kernel_in_front_does_not_run_the_waits_out(m):
     assert begin.elapsed_time(end) > 1500   # otherwise this shows nothing
     assert torch.equal(y, want)
     assert lib.sal_workspace_status(ws.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+
+
+@pytest.mark.parametrize("layout,m,k,n,q,g", [(0, 8, 20480, 256, 3, 128), (0, 3, 2080, 130, 3, 32), (0, 64, 4096, 264, 2, 64), (1, 16, 4096, 384, 3, 32),
+                                              (2, 9, 8192, 96, 2, 16)])
+def test_the_same_call_has_the_same_bits_whatever_the_scratch_grew_to(layout, m, k, n, q, g):
+    """Through a layer, a first call on a stream against the same call after a larger one, and through the C interface with the scratch that
+    the header asks for against more of it.  The split over CTAs decides the last bits."""
+    bits, alpha, _, x, bias = _case(layout, m, k, n, q, g)
+    lin = LutLinear(k, n, g if layout == 0 else 8 * g, q, bias=bias)
+    lin.binaryWeight, lin.alpha, lin.alpha_layout = bits, alpha, "row" if layout == 0 else "block"
+    torch.cuda.synchronize()
+    with torch.cuda.stream(torch.cuda.Stream()):
+        first = lin(x)
+        lin(x.repeat(200, 1)[:300])
+        assert torch.equal(lin(x), first)
+    torch.cuda.synchronize()
+    asked = _lib.load().sal_workspace_bytes(m, n)
+    ys = []
+    for size in (asked, 2 * asked, 1 << 28):
+        ws, y = torch.zeros(size, dtype=torch.uint8, device="cuda"), torch.empty(m, n, dtype=torch.float16, device="cuda")
+        assert _call(layout, bits, alpha, x, bias, y, k // g if layout == 0 else n // g, ws, size) == 0
+        ys.append(y)
+    assert torch.equal(ys[0], ys[1]) and torch.equal(ys[0], ys[2])
+
+
+def test_little_scratch_and_more_tiles_than_sms():
+    """Scratch for three CTAs where 150 column tiles have to be done: one CTA per tile."""
+    bits, alpha, mult, x, bias = _case(0, 16, 256, 150 * 128, 2, 128)
+    ref, bound = _reference(bits, mult, x, bias)
+    y = torch.empty(16, 150 * 128, dtype=torch.float16, device="cuda")
+    size = 16384 + 3 * 1024 * 16
+    ws = torch.zeros(size, dtype=torch.uint8, device="cuda")
+    assert _call(0, bits, alpha, x, bias, y, 2, ws, size) == 0
+    assert ((y.double() - ref).abs() <= bound).all() and not ws[256:].any()
