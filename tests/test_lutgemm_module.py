@@ -45,7 +45,7 @@ def test_compiled_module_exports_the_reference_names(module):
     shim.install()
 
 
-@pytest.mark.skipif(not os.path.isdir(REFERENCE), reason="the reference sources are not on this machine")
+@pytest.mark.skipif(not os.path.isfile(os.path.join(REFERENCE, "lut_gemm", "quant.py")), reason="the reference sources are not on this machine")
 def test_reference_lutlinear_imports_with_this_module_installed(module):
     """The unmodified reference module lut_gemm/quant.py does `import lutgemm` at import time
     (lut_gemm/quant.py:5); with this build installed it imports and constructs its LutLinear."""
@@ -104,7 +104,7 @@ def test_literal_reference_forward_call(module):
 
 
 @pytest.mark.gpu
-@pytest.mark.skipif(not os.path.isdir(REFERENCE), reason="the reference sources are not on this machine")
+@pytest.mark.skipif(not os.path.isfile(os.path.join(REFERENCE, "lut_gemm", "quant.py")), reason="the reference sources are not on this machine")
 def test_reference_lutlinear_forward_runs_on_this_build(module):
     """The reference's own LutLinear.forward, unmodified, on this build's kernels (square layer, int8 shifts
     written by hand: the reference's quantize_to_apot drops residual signs and emits 2**0 for exact powers of two)."""
