@@ -278,14 +278,14 @@ void sal_destroy_prepared(sal_prepared *prepared);
  * reaches `expected`, then clears it.  `workspace` may be NULL (no status reporting). */
 int sal_exchange_wait(void *local_flags, int slot, unsigned expected, void *workspace, void *stream);
 
-/* Introspection for tests and the benchmark: which kernel a mode-A call would
- * use (1 = tiled TMA kernel, 0 = generic) and its launch geometry. */
+/* Introspection for tests and the benchmark: which kernel a mode-A call of M rows would use, given aligned operands and
+ * scratch, and its launch geometry. */
 typedef struct sal_plan_info {
-    int tiled;
+    int tiled;       /* 1: tiled table kernel; 0: tensor-core kernel (several rows) if stages > 0, else generic kernel */
     int ctas;
-    int ranges;      /* column ranges */
-    int splits;      /* K splits */
-    int stages;
+    int ranges;      /* column ranges; tensor cores: output tiles (128 columns x up to 256 rows) */
+    int splits;      /* K splits; tensor cores: CTAs per tile, rounded up */
+    int stages;      /* depth of the ring of packed planes */
     int smem_bytes;
 } sal_plan_info;
 int sal_plan_shift_scale(int M, int K, int N, int q, int num_groups, sal_plan_info *out);

@@ -2018,19 +2018,26 @@ int sal_plan_shift_scale(int M, int K, int N, int q, int num_groups, sal_plan_in
     *out = sal_plan_info{};
     if (M < 1 || K <= 0 || N <= 0 || q < 1 || num_groups <= 0 || K % 32 || K % num_groups) return SAL_E_SHAPE;
     // alignment is assumed (fresh allocations are 256-byte aligned)
-    if (!tiled_eligible(reinterpret_cast<void *>(16), reinterpret_cast<void *>(16), nullptr, reinterpret_cast<void *>(16),
-                        nullptr, M, K, N, q, num_groups)) {
-        out->tiled = 0;
+    void *const any = reinterpret_cast<void *>(256);
+    const sal_problem sp = {any, any, nullptr, any, any, M, K, N, q, num_groups};
+    const bool tiled = tiled_eligible(any, any, nullptr, any, any, M, K, N, q, num_groups);
+    if (mma_wanted(&sp, 1, 0, sal_mma::ROW, tiled)) {
+        DeviceInfo *dev = nullptr;
+        sal_mma::Built b;
+        const int rc = sal_mma::build(&sp, 1, sal_mma::ROW, 0, (size_t)1 << 40, device_info(&dev) == SAL_OK ? dev->sms : 148, &b, false);
+        if (rc != SAL_OK) return rc;
+        out->ctas = b.ctas;
+        out->ranges = b.P.p[0].ntiles;
+        out->splits = b.P.whole_tiles ? 1 : (b.ctas + b.P.p[0].ntiles - 1) / b.P.p[0].ntiles;
+        out->stages = b.P.w_stages;
+        out->smem_bytes = b.smem;
+        return SAL_OK;
+    }
+    if (!tiled) {
         out->ctas = ((N + 127) / 128) * M;
         return SAL_OK;
     }
-    sal_problem sp = {};
-    sp.M = M;
-    sp.K = K;
-    sp.N = N;
-    sp.q = q;
-    sp.num_groups = num_groups;
-    return run_tiled_group(&sp, 1, 0, reinterpret_cast<void *>(16), (size_t)1 << 40, nullptr, out);
+    return run_tiled_group(&sp, 1, 0, any, (size_t)1 << 40, nullptr, out);
 }
 
 int sal_lutgemv_shift_scale(const void *bw, const void *alpha, const void *bias, const void *x, void *y, int M, int K,

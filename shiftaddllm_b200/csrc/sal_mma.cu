@@ -665,7 +665,7 @@ size_t full_scratch_bytes(int M) {
     return WS_PARTIALS + (size_t)MAX_CTAS * 2 * TILE_N * mt * sizeof(float);
 }
 
-int build(const sal_problem *problems, int count, AlphaLayout layout, unsigned flags, size_t ws_bytes, int sms, Built *out) {
+int build(const sal_problem *problems, int count, AlphaLayout layout, unsigned flags, size_t ws_bytes, int sms, Built *out, bool encode) {
     Built &b = *out;
     b = Built{};
     Params &P = b.P;
@@ -729,15 +729,15 @@ int build(const sal_problem *problems, int count, AlphaLayout layout, unsigned f
         if (tma_scales) {
             const int rows = layout == ROW ? (p.gw < UNIT_WORDS ? UNIT_WORDS / p.gw : 1) * b.q : 16 * b.q;
             p.s_tx = rows * P.s_pitch;
-            const int rc = sal_encode_rows(&p.smap, sp.alpha, layout == ROW ? sp.N : sp.num_groups, layout == ROW ? sp.num_groups * b.q : sp.K / 8 * b.q,
+            const int rc = !encode ? SAL_OK : sal_encode_rows(&p.smap, sp.alpha, layout == ROW ? sp.N : sp.num_groups, layout == ROW ? sp.num_groups * b.q : sp.K / 8 * b.q,
                                            P.s_pitch / 2, rows, 0);
             if (rc != SAL_OK) return rc;
         }
-        if (tma) {
+        if (tma && encode) {
             const int rc = sal_encode_planes(&p.tmap, sp.bw, sp.K, sp.N, sp.q, TILE_N, sp.q, UNIT_WORDS);
             if (rc != SAL_OK) return rc;
         }
-        if (!sp.x_mul) {
+        if (!sp.x_mul && encode) {
             const int rc = sal_encode_rows(&p.xmap, sp.x, sp.K, P.M, 64, P.mpad, 1);
             if (rc != SAL_OK) return rc;
         }

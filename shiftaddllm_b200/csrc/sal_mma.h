@@ -71,8 +71,9 @@ struct Built {
 
 // Can this product run here at all?
 bool eligible(const void *bw, const void *alpha, const void *x, int M, int K, int N, int q, int num_groups, AlphaLayout layout);
-// Plans one launch; `ws_bytes` of scratch will be there (0: none).  All problems share M, q and the layout.
-int build(const sal_problem *problems, int count, AlphaLayout layout, unsigned flags, size_t ws_bytes, int sms, Built *out);
+// Plans one launch; `ws_bytes` of scratch will be there (0: none).  All problems share M, q and the layout.  `encode`: also encode the
+// tensor maps (needs a CUDA context; false for a look at the plan only).
+int build(const sal_problem *problems, int count, AlphaLayout layout, unsigned flags, size_t ws_bytes, int sms, Built *out, bool encode = true);
 size_t scratch_bytes(const Built &b);   // 0: none
 // Scratch with which the split of a product of M rows (without x_mul) follows from its shape alone
 size_t full_scratch_bytes(int M);

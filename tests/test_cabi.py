@@ -129,3 +129,18 @@ def test_scratch_of_several_rows_holds_every_split():
         for n in (8, 130, 592, 4096):
             assert lib.sal_workspace_bytes(m, n) >= max(lib.sal_lutgemm_rows_workspace_bytes(m), 16384 + m * n * 64 * 4)
     assert lib.sal_lutgemm_rows_workspace_bytes(64) == 16384 + 148 * 2 * 128 * 64 * 4
+
+
+def test_plan_names_the_kernel_that_runs():
+    """Table, tensor-core and generic kernel by rows and shape; 4096 x 4096 with 8 rows is 32 column tiles, each shared by four CTAs."""
+    lib, info = _lib.load(), _lib.SalPlanInfo()
+
+    def kernel(m, k, n, q, groups):
+        assert lib.sal_plan_shift_scale(m, k, n, q, groups, ctypes.byref(info)) == 0
+        return "table" if info.tiled else "tensor" if info.stages else "generic"
+
+    assert [kernel(m, 4096, 4096, 3, 32) for m in (1, 6, 7, 64, 300)] == ["table", "table", "tensor", "tensor", "tensor"]
+    assert kernel(8, 4096, 4096, 3, 32) == "tensor" and (info.ctas, info.ranges, info.splits) == (128, 32, 4)
+    assert [kernel(m, 2080, 1378, 3, 65) for m in (1, 2)] == ["generic", "tensor"]
+    assert [kernel(8, 4096, 4096, q, 32) for q in (4, 5)] == ["tensor", "generic"]
+    assert kernel(600, 256, 64, 3, 1) == "tensor" and info.ranges == 3
