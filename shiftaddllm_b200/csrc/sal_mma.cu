@@ -47,6 +47,7 @@
 // does, before its first such wait.  The warps that issue copies and matrix instructions stop copying once they gave up, and wait (once more
 // bounded) for what they have in flight before the CTA ends; in a launch that ran as it should that has long been consumed.
 #include <cuda_fp16.h>
+#include <float.h>
 #include <stdint.h>
 
 #include <atomic>
@@ -250,11 +251,62 @@ __device__ __forceinline__ bool next_segment(const Params &P, int &u, int u_end,
 }
 
 template <int Q>
+__device__ float scaled_sums(const Params &P, const Problem &pr, int m, int n) {
+    const __half *x = reinterpret_cast<const __half *>(pr.x) + (size_t)m * pr.K;
+    float acc = 0.f;
+    for (int k = 0; k < pr.K / 32; k += pr.run)
+        for (int b = 0; b < Q; ++b) {
+            float sum = 0.f;
+            for (int r = 0; r < pr.run; ++r) {
+                const unsigned w = pr.bw[((size_t)(k + r) * Q + b) * pr.N + n];
+                for (int t = 0; t < 32; ++t) {
+                    const float v = __half2float(x[(k + r) * 32 + t]);
+                    sum += (w >> t) & 1u ? v : -v;
+                    if (P.layout != ROW && (t & 7) == 7) {   // a scale per eight features
+                        acc += __half2float(__ushort_as_half(pr.alpha[((size_t)(k * 4 + t / 8) * Q + b) * pr.ngroups + n / pr.gs])) * sum;
+                        sum = 0.f;
+                    }
+                }
+            }
+            if (P.layout == ROW) acc += __half2float(__ushort_as_half(pr.alpha[((size_t)(k / pr.gw) * Q + b) * pr.N + n])) * sum;
+        }
+    return acc;
+}
+
+// A scale that is infinite: the sum of (+-inf) * x over a group is NaN, while the table kernels, which multiply the signed sum of a group's
+// activations, give an infinity (NaN only if a column's infinite scales disagree).  All elements of such a column are no finite numbers, so a
+// CTA looks at one row's, and if one of them (for this or another reason) is none, goes over its tiles' scales and forms the elements of such
+// columns again in the tables' way.
+// `summed`: the tiles at the begin (bit 0) and end (bit 1) of the CTA's run that it was the last to arrive at.
+template <int Q>
+__device__ __noinline__ void infinite_columns(const Params &P, int summed) {
+    if (P.layout == BLOCK_U16) return;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int u, u_end;
+    cta_range(P, u, u_end);
+    Segment sg;
+    while (next_segment(P, u, u_end, sg)) {
+        const Problem &pr = P.p[sg.pi];
+        if (!(sg.k0 == 0 && sg.k1 == pr.ku) && !(summed & (sg.k0 == 0 ? 2 : 1))) continue;
+        const int rows = (P.layout == ROW ? pr.ngroups : pr.K / 8) * Q, pitch = P.layout == ROW ? pr.N : pr.ngroups;
+        for (int n = sg.n0 + warp; n < min(sg.n0 + TILE_N, pr.N); n += THREADS / 32) {
+            const unsigned short *scale = pr.alpha + (P.layout == ROW ? n : n / pr.gs);
+            bool any = false;
+#pragma unroll 8
+            for (int r = lane; r < rows; r += 32) any |= (scale[(size_t)r * pitch] & 0x7fffu) == 0x7c00u;
+            if (!__any_sync(0xffffffffu, any)) continue;
+            for (int m = sg.m0 + lane; m < sg.m0 + sg.rows; m += 32)   // no finite number, so bias and a finite y in place do not show
+                reinterpret_cast<__half *>(pr.y)[(size_t)m * pr.N + n] = __float2half_rn(scaled_sums<Q>(P, pr, m, n));
+        }
+    }
+}
+
+template <int Q>
 __global__ void __launch_bounds__(THREADS, 1) bcq_mma_kernel(const __grid_constant__ Params P) {
     using C = Cfg<Q>;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     __shared__ uint32_t s_tmem;
-    __shared__ int s_last;
+    __shared__ int s_last, s_summed, s_infinite;   // of the CTA's cut tiles: which it has summed; is an element no finite number?
     __shared__ __align__(8) uint64_t bars[2 * 16 + 3 * MAX_X_UNITS + 2 * 4 + 2];
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -273,6 +325,7 @@ __global__ void __launch_bounds__(THREADS, 1) bcq_mma_kernel(const __grid_consta
         fence_before();
     }
     if (tid == 0) {
+        s_summed = s_infinite = 0;
         for (int i = 0; i < P.w_stages; ++i) {
             // one arrival with the byte count of the TMA loads, and one per lane when its 4-byte copies have landed
             mbar_init(w_full + 8 * i, (P.use_tma ? 1 : 0) + (P.tma_scales ? 0 : 32));
@@ -474,7 +527,7 @@ __global__ void __launch_bounds__(THREADS, 1) bcq_mma_kernel(const __grid_consta
         const uint32_t tlane = tmem + ((uint32_t)(quarter * 32) << 16);
         int wst = 0, ast = wi >> 1;                                // words 0, 1: the first 64 features of a unit, 2, 3: the second
         uint32_t wph = 0, aph = 1, dph = 0;
-        bool waited = false;
+        bool waited = false, finite = true;
         while (next_segment(P, u, u_end, sg)) {
             const Problem &pr = P.p[sg.pi];
             const int gw = pr.gw, gshift = pr.gshift;
@@ -553,6 +606,7 @@ __global__ void __launch_bounds__(THREADS, 1) bcq_mma_kernel(const __grid_consta
             for (int m = m_lo; m < m_hi; m += 4) {
                 float v[4];
                 tmem_load4(tlane + m, v);
+                if (m == 0 && whole) finite = finite && fabsf(v[0]) <= FLT_MAX;   // one row shows it
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     if (m + i < m_hi) {
@@ -604,6 +658,7 @@ __global__ void __launch_bounds__(THREADS, 1) bcq_mma_kernel(const __grid_consta
 #pragma unroll
                                 for (int i = 0; i < 2; ++i) v[i].x += t[c][i].x, v[i].y += t[c][i].y, v[i].z += t[c][i].z, v[i].w += t[c][i].w;
                         }
+                        if (m == 0) finite = finite && fabsf(v[0].x) <= FLT_MAX && fabsf(v[0].y) <= FLT_MAX && fabsf(v[0].z) <= FLT_MAX && fabsf(v[0].w) <= FLT_MAX;
 #pragma unroll
                         for (int i = 0; i < 2; ++i) {
                             const int mm = m + i * OP_WARPS;
@@ -619,9 +674,11 @@ __global__ void __launch_bounds__(THREADS, 1) bcq_mma_kernel(const __grid_consta
                                 }
                         }
                     }
+                    if (tid == 0) s_summed |= sg.k0 == 0 ? 2 : 1;
                 }
             }
         }
+        if (!finite) s_infinite = 1;
         fence_before();
     }
     __syncthreads();
@@ -629,6 +686,7 @@ __global__ void __launch_bounds__(THREADS, 1) bcq_mma_kernel(const __grid_consta
         fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
     }
+    if (s_infinite) infinite_columns<Q>(P, s_summed);
 }
 
 template <int Q>
@@ -702,6 +760,7 @@ int build(const sal_problem *problems, int count, AlphaLayout layout, unsigned f
         p.bw = reinterpret_cast<const unsigned *>(sp.bw);
         p.alpha = reinterpret_cast<const unsigned short *>(sp.alpha);
         p.bias = reinterpret_cast<const unsigned short *>(sp.bias);
+        p.x = reinterpret_cast<const unsigned short *>(sp.x);
         p.y = reinterpret_cast<unsigned short *>(sp.y);
         p.K = sp.K, p.N = sp.N;
         p.ku = (sp.K + 127) / 128;
@@ -713,9 +772,10 @@ int build(const sal_problem *problems, int count, AlphaLayout layout, unsigned f
         units += p.ntiles * p.ku;
         tiles += p.ntiles;
         p.ngroups = sp.num_groups;
-        p.gw = 1, p.gshift = 0, p.gs = 1;
+        p.gw = 1, p.gshift = 0, p.gs = 1, p.run = 1;
         if (layout == ROW) {
             p.gw = sp.K / sp.num_groups / 32;
+            p.run = sp.K % 256 == 0 && sp.N % 8 == 0 && p.gw % 4 == 0 ? 4 : 1;   // the tiled table kernel's shapes, else the generic one's
             // groups that a unit of four words can meet: one if they are whole units
             const int ng = p.gw % UNIT_WORDS == 0 ? 1 : (UNIT_WORDS - 2) / p.gw + 2;
             if (ng * b.q * P.s_pitch > P.s_bytes) P.s_bytes = ng * b.q * P.s_pitch;
@@ -818,6 +878,7 @@ int launch(const Built &b, void *workspace, size_t ws_bytes, cudaStream_t stream
         // silu(x) * x_mul, formed once in front of the product (every column tile reads it)
         const int rc = sal_silu_mul_f16(b.gate[i], b.up[i], base + off, P.M * P.p[i].K, stream);
         if (rc != SAL_OK) return rc;
+        P.p[i].x = reinterpret_cast<const unsigned short *>(base + off);
         const int erc = sal_encode_rows(&P.p[i].xmap, base + off, P.p[i].K, P.M, 64, P.mpad, 1);
         if (erc != SAL_OK) return erc;
         off += ((size_t)P.M * P.p[i].K * 2 + 255) & ~(size_t)255;

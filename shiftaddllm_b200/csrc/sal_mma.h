@@ -25,8 +25,10 @@ struct Problem {
     const unsigned *bw;
     const unsigned short *alpha;
     const unsigned short *bias;
+    const unsigned short *x;
     unsigned short *y;
     int K, N;
+    int run;          // ROW: words whose sum the table kernels multiply by a scale at a time
     int s_tx;         // bytes of scales per unit by TMA
     int ku;           // 128-feature units of K
     int unit_begin;   // first unit of the problem in the launch's unit sequence

@@ -194,3 +194,23 @@ def test_little_scratch_and_more_tiles_than_sms():
     ws = torch.zeros(size, dtype=torch.uint8, device="cuda")
     assert _call(0, bits, alpha, x, bias, y, 2, ws, size) == 0
     assert ((y.double() - ref).abs() <= bound).all() and not ws[256:].any()
+
+
+@pytest.mark.parametrize("layout,m,k,n,q,g", [(0, 8, 2048, 264, 3, 128), (0, 40, 512, 128, 2, 512), (0, 5, 2080, 130, 3, 32), (0, 300, 512, 64, 4, 256),
+                                              (1, 9, 1024, 144, 3, 16), (1, 70, 288, 768, 2, 48)])
+def test_infinite_and_nan_operands_as_in_the_tables(layout, m, k, n, q, g):
+    """Infinite scales, alone and several in a column, NaN scales, and infinite and NaN activations: where a row of one gives an infinity (of
+    which sign) or NaN, so do many; everywhere else the elements stay within the bound.  `m` rows are tensor-core work, one row is the tables'."""
+    bits, alpha, mult, x, bias = _case(layout, m, k, n, q, g)
+    ref, bound = _reference(bits, mult, x, bias)
+    inf, nan = float("inf"), float("nan")
+    alpha[0, 0, 1], alpha[-1, q - 1, 2], alpha[0, q - 1, 3], alpha[-1, 0, 3], alpha[0, 0, 5] = inf, -inf, inf, inf, nan
+    x[1, 7], x[2, k - 1], x[3, 11] = inf, -inf, nan
+    lin = LutLinear(k, n, g if layout == 0 else 8 * g, q, bias=bias)
+    lin.binaryWeight, lin.alpha, lin.alpha_layout = bits, alpha, "row" if layout == 0 else "block"
+    got, want = lin(x), torch.cat([lin(x[i:i + 1]) for i in range(m)])
+    assert torch.equal(got.isnan(), want.isnan())
+    assert torch.equal(torch.where(got.isinf(), got, 0), torch.where(want.isinf(), want, 0))
+    finite = got.isfinite()
+    assert finite.sum() >= (m - 3) * n // 2 and got.isinf().any() and got.isnan().any()
+    assert ((got.double() - ref).abs() <= bound)[finite].all()
