@@ -1818,21 +1818,35 @@ int run_tiled_group(const sal_problem *problems, int count, unsigned flags, void
 }
 
 // Products of several activation rows go to the tensor cores (sal_mma.cu) from this many rows on.  There the time hardly depends on the
-// rows, here it is a pass over all lookups per pair of rows (ROW; per row in the block layouts).  Times in us for 2 / 4 / 6 / 8 / 16 rows,
-// 4096 x 11008, 4 planes: tables 15 / 20 / 27 / 31 / 54, tensor cores 27 at all of them; 28672 x 8192, 2 planes: 32 / 45 / 58 / 74 / 132
-// against 70; block layout (16 columns), 4096 x 4096, 3 planes, 3 / 4 / 8 rows: 15 / 18 / 30 against 16.  Shapes that the tiled
-// table kernel does not take ran on the generic one, row by row: 2080 x 1378, 3 planes, 3 rows, 21 against 18.
+// rows, here it is a pass over all lookups per pair of rows (ROW; per row in the block layouts).  Times in us, tables / tensor cores, in a
+// CUDA graph, weights from HBM:
+//   ROW, 4 / 6 / 8 / 16 rows: 4096 x 11008, 4 planes 23 / 30 / 34 / 58 against 30; 28672 x 8192, 2 planes 43 / 60 / 77 / 132 against 79; 8192 x
+//   28672, 2 planes, 6 / 8 rows 61 / 78 against 74; 4096 x 4096, 3 planes 15 / 17 / 19 / 24 against 15.  Seven and eight rows lose up to 5 % at the
+//   largest K with few planes, and up to 2 us where the tables' launch is one wave of short CTAs (3072 x 768, 3 planes: 9.1 / 10.9); they go to
+//   the tensor cores all the same, since the pairs' tables hold fp16 entries: an error of 4.3e-4 against 2.1e-4, the rounding of the result.
+//   Block layouts hold fp32 entries, so there the line is a matter of time alone: see block_tables_us.
+//   Shapes that the tiled table kernel does not take ran on the generic one, row by row: 2080 x 1378, 3 planes, 3 rows 23 / 17.
 #ifdef SAL_MEASURE
 int g_mma_min_rows = 7, g_mma_min_rows_block = 4, g_mma_min_rows_generic = 2;
 #else
 constexpr int g_mma_min_rows = 7, g_mma_min_rows_block = 4, g_mma_min_rows_generic = 2;
 #endif
+// Estimated time in us of a block-layout product on the tables: in one wave of CTAs (two to an SM) nearly constant, then by the lookups.  With
+// sal_mma::block_us it was within 0.5 % on average of the better choice, 17 % at worst, over 489 measured (shape, planes, rows) from 512 x 512
+// to 28672 x 8192, 4 to 64 rows; always taking the tensor cores from four rows on lost 6 % on average and 47 % at worst (2048 x 512, 3 planes, 4 rows:
+// 8.5 / 10.8; 4096 x 4096, 3 planes, 4 rows 20.2 / 17.0; 2048 x 2048, 3 planes, 4 / 5 rows 10.6 / 10.9 and 13.1 / 11.0).
+double block_tables_us(const sal_problem &p, int sms) {
+    static const double base[4] = {6.6, 7.4, 8.5, 8.9}, unit[4] = {0.6, 0.93, 1.6, 2.1};
+    const double u = (double)p.M * (p.K / KB_FEATS) * ((p.N + 255) / 256) / sms;   // 256 x 256 blocks of weights per SM
+    return base[p.q - 1] + (u <= 1.0 ? 0.0 : u <= 2.0 ? 1.8 : 0.6 + unit[p.q - 1] * u);
+}
 bool mma_wanted(const sal_problem *problems, int count, unsigned flags, sal_mma::AlphaLayout layout, bool tiled) {
     if (flags & (SAL_FORCE_GENERIC | SAL_OUT_FIXED_ATOMIC | SAL_SWIGLU_FIXED)) return false;
     const int min_rows = !tiled ? g_mma_min_rows_generic : layout == sal_mma::ROW ? g_mma_min_rows : g_mma_min_rows_block;
     for (int i = 0; i < count; ++i) {
         const sal_problem &p = problems[i];
         if (p.M < min_rows || !sal_mma::eligible(p.bw, p.alpha, p.x, p.M, p.K, p.N, p.q, p.num_groups, layout)) return false;
+        if (tiled && layout != sal_mma::ROW && block_tables_us(p, 148) < 0.98 * sal_mma::block_us(p, layout, 148)) return false;
     }
     return true;
 }

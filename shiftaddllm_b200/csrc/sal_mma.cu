@@ -709,7 +709,44 @@ cudaError_t launch_q(const Built &b, const Params &P, cudaStream_t stream) {
     return cudaLaunchKernelEx(&cfg, bcq_mma_kernel<Q>, P);
 }
 
+// CTAs per tile where all CTAs have the same number of them (0: runs of units are cut anywhere).
+// Where whole numbers of shares per tile fill most of the SMs, runs are cut at tile borders (run_begin does so by itself): every
+// CTA has one segment instead of two, and a tile fewer shares to sum, which for many rows costs as much as the product.  At least
+// four units per share, or eight shares.  us with 148 CTAs / with whole shares, for 64 and 256 rows: 4096 x 4096, 3 planes 20.3 / 17.3
+// and 43.3 / 36.2 (128 CTAs), 4096 x 1024 15.3 / 13.5 and 45.4 / 32.3 (64), 2048 x 2048 14.8 / 11.2 and 37.7 / 29.2 (128), 8192 x 8192,
+// 2 planes 32.7 / 32.0 and 70.2 / 73.1 (128); with 86 of 148 (4096 x 11008) 36.7 / 45.8, hence the line at 86 %.
+// Not where rows are copied by plain instructions: a unit takes three times as long there (2080 x 1378, 3 rows: 18.4 / 20.5).
+int whole_shares(int tiles, int ku, int sms) {
+    if (tiles > sms) return 0;
+    const int most = ku / 4 > 8 ? ku / 4 : 8;
+    int shares = sms / tiles;
+    const bool enough = shares > most;
+    if (shares > most) shares = most;
+    if (shares > ku) shares = ku;
+    return enough || shares * tiles * 100 >= 86 * sms ? shares : 0;
+}
+
+// Can the scales be fetched by TMA?  Rows of a multiple of 16 bytes; ROW: groups that make a unit or that a unit is made of, BLOCK: eight
+// groups per tile.
+bool scales_by_tma(const sal_problem &sp, AlphaLayout layout) {
+    const int gw = layout == ROW ? sp.K / sp.num_groups / 32 : 0;
+    return (layout == ROW ? sp.N : sp.num_groups) % 8 == 0 && (reinterpret_cast<uintptr_t>(sp.alpha) & 15) == 0 &&
+           (layout == ROW ? gw % UNIT_WORDS == 0 || UNIT_WORDS % gw == 0 : sp.N / sp.num_groups == 16);
+}
+bool planes_by_tma(const sal_problem &sp) { return sp.N % 4 == 0 && (reinterpret_cast<uintptr_t>(sp.bw) & 15) == 0; }
+
 }  // namespace
+
+double block_us(const sal_problem &sp, AlphaLayout layout, int sms) {
+    if (sms > MAX_CTAS) sms = MAX_CTAS;
+    const int ku = (sp.K + 127) / 128, tiles = (sp.N + TILE_N - 1) / TILE_N * ((sp.M + MAX_MT - 1) / MAX_MT), i = sp.q - 1;
+    const bool tma = planes_by_tma(sp) && scales_by_tma(sp, layout);
+    const int shares = tma ? whole_shares(tiles, ku, sms) : 0, ctas = shares ? shares * tiles : (sms < tiles * ku ? sms : tiles * ku);
+    static const double by_tma[4] = {0.45, 0.72, 1.03, 1.28}, by_copies[4] = {0.7, 1.0, 1.38, 1.56};
+    double unit = tma ? by_tma[i] * (shares ? 1.0 : tiles > sms ? 1.06 : 1.2) : by_copies[i];
+    if (layout == BLOCK_U16) unit *= tma ? 1.3 : 1.1;   // decoding the exponents
+    return (tma ? 8.2 : 11.0) + unit * ((tiles * ku + ctas - 1) / ctas) + 0.06 * shares + (sp.M > 16 ? 0.06 * (sp.M - 16) : 0.0);
+}
 
 bool eligible(const void *bw, const void *alpha, const void *x, int M, int K, int N, int q, int num_groups, AlphaLayout layout) {
     if (M < 1 || M > MAX_ROWS || q < 1 || q > 4 || K < 32 || K % 32 || N < 1 || num_groups < 1) return false;
@@ -738,18 +775,10 @@ int build(const sal_problem *problems, int count, AlphaLayout layout, unsigned f
     P.accumulate = (flags & SAL_ACCUMULATE) ? 1 : 0;
     P.layout = layout;
     bool tma = true;
-    for (int i = 0; i < count; ++i)
-        if (problems[i].N % 4 || (reinterpret_cast<uintptr_t>(problems[i].bw) & 15)) tma = false;
+    for (int i = 0; i < count; ++i) tma = tma && planes_by_tma(problems[i]);
     P.use_tma = tma;
-    // scales by TMA: rows of a multiple of 16 bytes; ROW: groups that make a unit or that a unit is made of, BLOCK: eight groups per tile
     bool tma_scales = tma;
-    for (int i = 0; i < count; ++i) {
-        const sal_problem &sp = problems[i];
-        const int gw = layout == ROW ? sp.K / sp.num_groups / 32 : 0;
-        if ((layout == ROW ? sp.N : sp.num_groups) % 8 || (reinterpret_cast<uintptr_t>(sp.alpha) & 15) ||
-            (layout == ROW ? gw % UNIT_WORDS != 0 && UNIT_WORDS % gw != 0 : sp.N / sp.num_groups != 16))
-            tma_scales = false;
-    }
+    for (int i = 0; i < count; ++i) tma_scales = tma_scales && scales_by_tma(problems[i], layout);
     P.tma_scales = tma_scales;
     P.s_pitch = layout == ROW ? (tma_scales ? S_PITCH_ROW_TMA : S_PITCH_ROW) : (tma_scales ? S_PITCH_BLOCK_TMA : S_PITCH_BLOCK);
     int units = 0, tiles = 0;
@@ -809,25 +838,12 @@ int build(const sal_problem *problems, int count, AlphaLayout layout, unsigned f
     // CTAs: one per SM, as far as there are units and the scratch buffer holds their partial sums (two slots of mt x 128
     // floats each; the documented size holds them all, so that the split and with it the last bits follow from the shape alone);
     // without scratch, or with so little that it would leave SMs idle, one per output tile
-    // Where whole numbers of shares per tile fill most of the SMs, runs are cut at tile borders (run_begin does so by itself): every
-    // CTA has one segment instead of two, and a tile fewer shares to sum, which for many rows costs as much as the product.  At least
-    // four units per share, or eight shares.  us with 148 CTAs / with whole shares, for 64 and 256 rows: 4096 x 4096, 3 planes 20.3 / 17.3
-    // and 43.3 / 36.2 (128 CTAs), 4096 x 1024 15.3 / 13.5 and 45.4 / 32.3 (64), 2048 x 2048 14.8 / 11.2 and 37.7 / 29.2 (128), 8192 x 8192,
-    // 2 planes 32.7 / 32.0 and 70.2 / 73.1 (128); with 86 of 148 (4096 x 11008) 36.7 / 45.8, hence the line at 86 %.
-    // Not where rows are copied by plain instructions: a unit takes three times as long there (2080 x 1378, 3 rows: 18.4 / 20.5).
     const size_t slot_bytes = (size_t)2 * P.mt * TILE_N * sizeof(float);
     if (sms > MAX_CTAS) sms = MAX_CTAS;
-    long long ctas = sms < units ? sms : units;
     bool same_k = true;
     for (int i = 1; i < count; ++i) same_k = same_k && P.p[i].ku == P.p[0].ku;
-    if (same_k && tma_scales && tiles <= sms) {
-        const int ku = P.p[0].ku, most = ku / 4 > 8 ? ku / 4 : 8;
-        int shares = sms / tiles;
-        const bool enough = shares > most;
-        if (shares > most) shares = most;
-        if (shares > ku) shares = ku;
-        if (enough || shares * tiles * 100 >= 86 * sms) ctas = (long long)shares * tiles;
-    }
+    const int shares = same_k && tma_scales ? whole_shares(tiles, P.p[0].ku, sms) : 0;
+    long long ctas = shares ? (long long)shares * tiles : (sms < units ? sms : units);
     if (ws_bytes < WS_PARTIALS + b.act_bytes) {
         if (b.act_bytes) return SAL_E_WORKSPACE;
         ctas = 0;

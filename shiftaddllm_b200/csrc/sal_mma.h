@@ -73,6 +73,8 @@ struct Built {
 
 // Can this product run here at all?
 bool eligible(const void *bw, const void *alpha, const void *x, int M, int K, int N, int q, int num_groups, AlphaLayout layout);
+// Estimated time in us of a product in one of the BLOCK layouts (see block_tables_us in sal_lutgemm.cu).
+double block_us(const sal_problem &problem, AlphaLayout layout, int sms);
 // Plans one launch; `ws_bytes` of scratch will be there (0: none).  All problems share M, q and the layout.  `encode`: also encode the
 // tensor maps (needs a CUDA context; false for a look at the plan only).
 int build(const sal_problem *problems, int count, AlphaLayout layout, unsigned flags, size_t ws_bytes, int sms, Built *out, bool encode = true);

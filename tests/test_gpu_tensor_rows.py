@@ -5,6 +5,8 @@ shared by many CTAs or none, and the scratch limits that change the split.
 Reference: the same product in float64.  Bound per element: the output's fp16 rounding (2**-11 of the value, or half the smallest
 subnormal) plus one fp32 rounding (2**-23, which also covers truncation) per accumulation step, of which a tile has K * q / 16 and the
 sum over CTAs at most 64, each of at most the sum of the magnitudes."""
+import ctypes
+
 import pytest
 import torch
 
@@ -214,3 +216,41 @@ def test_infinite_and_nan_operands_as_in_the_tables(layout, m, k, n, q, g):
     finite = got.isfinite()
     assert finite.sum() >= (m - 3) * n // 2 and got.isinf().any() and got.isnan().any()
     assert ((got.double() - ref).abs() <= bound)[finite].all()
+
+
+def _block_sizes(fn):
+    """Threads per block of the kernels that `fn` enqueues."""
+    drv, stream, graph, count = ctypes.CDLL("libcuda.so.1"), torch.cuda.Stream(), ctypes.c_void_p(), ctypes.c_size_t()
+    with torch.cuda.stream(stream):
+        fn()
+        torch.cuda.synchronize()
+        assert drv.cuStreamBeginCapture_v2(ctypes.c_void_p(stream.cuda_stream), 1) == 0
+        fn()
+        assert drv.cuStreamEndCapture(ctypes.c_void_p(stream.cuda_stream), ctypes.byref(graph)) == 0
+    assert drv.cuGraphGetNodes(graph, None, ctypes.byref(count)) == 0
+    nodes = (ctypes.c_void_p * count.value)()
+    assert drv.cuGraphGetNodes(graph, nodes, ctypes.byref(count)) == 0
+    sizes = []
+    for node in nodes:
+        params = (ctypes.c_uint32 * 32)()   # CUDA_KERNEL_NODE_PARAMS: function, grid x y z, block x y z, ..
+        assert drv.cuGraphKernelNodeGetParams_v2(ctypes.c_void_p(node), params) == 0
+        sizes.append(params[5])
+    assert drv.cuGraphDestroy(graph) == 0
+    return sizes
+
+
+@pytest.mark.parametrize("layout,m,k,n,q,g,tensor", [(1, 4, 768, 768, 3, 16, False), (1, 4, 2048, 512, 3, 16, False), (1, 32, 768, 768, 3, 16, False),
+                                                     (1, 6, 2048, 2048, 3, 16, True), (1, 6, 2048, 2048, 3, 128, False), (1, 4, 11008, 4096, 3, 16, True),
+                                                     (2, 4, 4096, 4096, 2, 128, False), (1, 3, 4096, 4096, 4, 16, False), (1, 64, 512, 2048, 2, 16, True)])
+def test_block_layouts_run_where_they_are_faster(layout, m, k, n, q, g, tensor):
+    """The table kernel has 288 threads, the tensor-core kernel 736; both within the bound on either side of the line."""
+    bits, alpha, mult, x, bias = _case(layout, m, k, n, q, g)
+    ref, bound = _reference(bits, mult, x, bias)
+    y = torch.empty(m, n, dtype=torch.float16, device="cuda")
+
+    def call():
+        lutgemm.lutgemm_block_fused(y, bits, alpha, bias, x, n, k, q, n // g)
+
+    assert _block_sizes(call) == [736 if tensor else 288]
+    call()
+    assert ((y.double() - ref).abs() <= bound).all()
