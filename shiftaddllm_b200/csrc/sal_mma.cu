@@ -606,7 +606,7 @@ __global__ void __launch_bounds__(THREADS, 1) bcq_mma_kernel(const __grid_consta
             for (int m = m_lo; m < m_hi; m += 4) {
                 float v[4];
                 tmem_load4(tlane + m, v);
-                if (m == 0 && whole) finite = finite && fabsf(v[0]) <= FLT_MAX;   // one row shows it
+                if (m == 0 && whole && n < pr.N) finite = finite && fabsf(v[0]) <= FLT_MAX;   // one row shows it
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     if (m + i < m_hi) {
@@ -658,7 +658,11 @@ __global__ void __launch_bounds__(THREADS, 1) bcq_mma_kernel(const __grid_consta
 #pragma unroll
                                 for (int i = 0; i < 2; ++i) v[i].x += t[c][i].x, v[i].y += t[c][i].y, v[i].z += t[c][i].z, v[i].w += t[c][i].w;
                         }
-                        if (m == 0) finite = finite && fabsf(v[0].x) <= FLT_MAX && fabsf(v[0].y) <= FLT_MAX && fabsf(v[0].z) <= FLT_MAX && fabsf(v[0].w) <= FLT_MAX;
+                        if (m == 0) {   // columns past N have whatever scales the ring held
+                            const float r0[4] = {v[0].x, v[0].y, v[0].z, v[0].w};
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) finite = finite && (nc + e >= pr.N || fabsf(r0[e]) <= FLT_MAX);
+                        }
 #pragma unroll
                         for (int i = 0; i < 2; ++i) {
                             const int mm = m + i * OP_WARPS;
