@@ -12,13 +12,15 @@ reference, so kernel-format state dicts load unchanged.  The dtype of
   — the literal call of the reference's ``forward`` (lut_gemm/quant.py:50-51)
 
 Extensions that do not break the above: ``bias=None`` works (LLaMA has no
-bias), inputs may hold up to 64 rows per call (longer inputs are chunked),
-and the bias add is fused into the kernel.
+bias), inputs may hold any number of rows (one launch takes up to 4096 of
+them on the tensor cores, 64 where those do not take the layer), and the bias
+add is fused into the kernel.
 """
 from __future__ import annotations
 
 import math
 import os
+import warnings
 
 import torch
 import torch.nn as nn
@@ -27,7 +29,7 @@ from . import lutgemm
 
 APOT_NONE = -128
 
-_native = None   # the compiled module's lut_linear; False where the module has not been built
+_native = None   # the compiled module's lut_linear; False where the module has not been built or cannot be imported
 
 
 def _native_linear():
@@ -38,7 +40,12 @@ def _native_linear():
 
         _lib = lutgemm._lib
         _lib.load()   # the module links to the library by name: the one loaded here (SAL_LUTGEMM_LIBRARY) is the one it finds
-        _native = getattr(lutgemm.compiled_module(), "lut_linear", False) if os.path.exists(build.extension_path()) else False
+        _native = False
+        if os.path.exists(build.extension_path()):
+            try:
+                _native = getattr(lutgemm.compiled_module(), "lut_linear", False)
+            except (ImportError, OSError) as e:   # built for another interpreter or torch: `forward` does without it
+                warnings.warn(f"the compiled module cannot be imported, LutLinear.forward takes its steps in Python: {e}")
     return _native
 
 

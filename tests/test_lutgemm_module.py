@@ -4,6 +4,7 @@ import importlib
 import os
 import sys
 import types
+import warnings
 
 import numpy as np
 import pytest
@@ -133,3 +134,52 @@ def test_reference_lutlinear_forward_runs_on_this_build(module):
         sys.path.remove(REFERENCE)
         for name in [n_ for n_ in sys.modules if n_ == "lut_gemm" or n_.startswith("lut_gemm.")]:
             del sys.modules[name]
+
+
+def test_forward_does_without_a_module_that_cannot_be_imported(monkeypatch):
+    """A module file built for another torch or interpreter: `forward` takes its steps in Python, with one warning."""
+    from shiftaddllm_b200 import quant
+
+    def broken():
+        raise ImportError("undefined symbol")
+
+    monkeypatch.setattr(shim, "compiled_module", broken)
+    monkeypatch.setattr(build, "extension_path", lambda: __file__)
+    monkeypatch.setattr(quant, "_native", None)
+    with pytest.warns(UserWarning, match="undefined symbol"):
+        assert quant._native_linear() is False
+    with warnings.catch_warnings():
+        warnings.simplefilter("error")
+        assert quant._native_linear() is False
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["row", "block_f16", "block_i16", "block_i8"])
+def test_forward_in_native_code_and_in_python(kind, monkeypatch):
+    """The same layer through the compiled module and through the Python steps: same bits up to 64 rows, beyond (one launch against one per 64
+    rows) within the rounding of the result."""
+    from shiftaddllm_b200 import quant
+
+    k, n, q = 512, 256, 3
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    lin = quant.LutLinear(k, n, 128, q, bias=torch.nn.Parameter(0.1 * torch.randn(n, device="cuda", generator=gen)))
+    lin.binaryWeight = torch.randint(-2 ** 31, 2 ** 31, (k // 32, q, n), dtype=torch.int32, device="cuda", generator=gen)
+    if kind == "row":
+        lin.set_row_alpha(torch.rand(k // 128, q, n, device="cuda", generator=gen))
+    elif kind == "block_i16":
+        lin.alpha, lin.alpha_layout = torch.randint(0, 512, (k // 8, q, n // 16), device="cuda", generator=gen).to(torch.int16), "block"
+    else:
+        lin.set_block_alpha(torch.exp2(-torch.randint(2, 9, (k // 8, q, n // 16), device="cuda", generator=gen).float()), apot=kind == "block_i8")
+    wide = torch.randn(130, 2 * k, device="cuda", generator=gen)
+    inputs = [wide[:0, :k].half(), wide[:1, :k], wide[:5, ::2].half(), wide[:64, k:].half().view(4, 16, k), wide[0, :k].bfloat16(), wide[:, :k].half()]
+    assert quant._native_linear()
+    with torch.no_grad():
+        native = [lin(x) for x in inputs]
+        monkeypatch.setattr(quant, "_native", False)
+        for x, a in zip(inputs, native):
+            b = lin(x)
+            assert a.dtype == b.dtype == x.dtype and a.shape == b.shape == (*x.shape[:-1], n)
+            if x.numel() <= 64 * k:
+                assert torch.equal(a, b)
+            else:
+                assert (a.float() - b.float()).norm() <= 2.0 ** -10 * b.float().norm()
