@@ -272,37 +272,36 @@ class BcqLlamaDecoder:
         self.k_cache.zero_()
         self.v_cache.zero_()
 
-    def feed(self, token_ids, chunk: int = 64):
-        """Teacher-forced pass over a prompt (fills the KV cache).  `chunk` > 1: the prompt goes through the
-        model in chunks of up to `chunk` (at most 64) tokens, every linear layer as ONE small-batch LUT product
-        per chunk — the way the reference feeds a prompt through the model's ordinary forward
-        (model/opt.py:397-411) — instead of one decode step per token.  `chunk` = 1: one step (graph replay)
-        per token."""
-        if chunk > 1 and len(token_ids) > 1:
+    def feed(self, token_ids, chunk: int | None = None):
+        """Teacher-forced pass over a prompt (fills the KV cache): through the model in passes of many tokens (`prefill`, which also says
+        what `chunk` bounds), every linear layer as one product per pass — the way the reference feeds a prompt through the model's
+        ordinary forward (model/opt.py:397-411) — instead of one decode step per token.  `chunk` = 1: one step (graph replay) per token."""
+        if (chunk is None or chunk > 1) and len(token_ids) > 1:
             return self.prefill(token_ids, chunk)
         run = self.graph.replay if self.graph is not None else self.step
         for t in token_ids:
             self.token.fill_(int(t))
             run()
 
-    PREFILL_ROWS = 512   # prompt rows of one pass (`prefill`): two full row tiles of the tensor-core product
+    PREFILL_ROWS = 512   # prompt rows of one pass (`prefill`) if the caller names no bound: two full row tiles of the tensor-core product
 
-    def prefill(self, token_ids, chunk: int = 64):
+    def prefill(self, token_ids, chunk: int | None = None):
         """Prompt pass: the rows of a pass share each weight stream (one product per layer and pass; a last pass of one
-        token runs the M = 1 kernel).  `chunk` below 64 bounds the rows of a pass; from 64 on passes of
-        up to PREFILL_ROWS are taken where the layers allow it (the result does not depend on it beyond rounding).  Between the
-        products: residual + RMSNorm, rotary step + cache write and causal softmax are one helper launch each, the two attention
-        products torch's batched matmul.  Leaves the cache, `pos`, the logits of the last prompt token and the greedy next token
+        token runs the M = 1 kernel).  A pass has at most `chunk` rows (None: PREFILL_ROWS), and at most 64 where a layer has more than
+        four planes; the result does not depend on it beyond rounding.  The scores of a pass take heads x rows x positions fp16
+        numbers, so `chunk` also bounds memory.  Between the products: residual + RMSNorm, rotary step + cache write and causal softmax
+        are one helper launch each, the two attention products torch's batched matmul.  Leaves the cache, `pos`, the logits of the last prompt token and the greedy next token
         exactly where a token-by-token `feed` would."""
         s = self.shape
         hd, kvh, rep, h = s.head_dim, s.kv_heads, s.heads // s.kv_heads, s.hidden
-        chunk = max(1, min(int(chunk), 64))
+        rows = min(self.PREFILL_ROWS if chunk is None else max(1, int(chunk)), lutgemm._lib.SAL_MAX_ROWS)
+        if any(l.wbit > 4 for b in self.blocks for l in b.linears().values()):
+            rows = min(rows, lutgemm._lib.SAL_MAX_M)    # the tables' limit; the tensor-core product takes up to four planes
+        many = rows > lutgemm._lib.SAL_MAX_M
         ids = torch.as_tensor(token_ids, dtype=torch.long, device=self.device).view(-1)
         p0 = int(self.pos.item())
         if p0 + ids.numel() > self.max_len:
             raise ValueError("prompt does not fit the KV cache")
-        many = chunk == 64 and all(l.wbit <= 4 for b in self.blocks for l in b.linears().values())
-        rows = self.PREFILL_ROWS if many else chunk
         f16 = dict(dtype=torch.float16, device=self.device)
         scale = 1.0 / math.sqrt(hd)
         for c0 in range(0, ids.numel(), rows):

@@ -67,3 +67,15 @@ def test_prompt_of_several_passes(chunk, monkeypatch):
     # two layers' chain of eight roundings with headroom for the logits' sum over the hidden size
     for got, ref in zip((model.logits, model.k_cache, model.v_cache), want):
         assert (got.float() - ref).norm() <= 8 * 2.0 ** -9 * ref.norm()
+
+
+@pytest.mark.parametrize("chunk,passes", [(64, [64, 64, 22]), (63, [63, 63, 24]), (100, [100, 50]), (None, [70, 70, 10]), (1000, [150])])
+def test_chunk_is_the_bound_on_the_rows_of_a_pass(chunk, passes, monkeypatch):
+    from shiftaddllm_b200 import decoder
+
+    rows, group = [], decoder._group
+    monkeypatch.setattr(BcqLlamaDecoder, "PREFILL_ROWS", 70)
+    monkeypatch.setattr(decoder, "_group", lambda lins, x, *a, **k: (rows.append(x.shape[0]), group(lins, x, *a, **k))[1])
+    model = BcqLlamaDecoder(SHAPES["tiny"], 3, 128, max_len=160)
+    model.feed(list(range(150)), **({} if chunk is None else {"chunk": chunk}))
+    assert rows[::4 * SHAPES["tiny"].layers] == passes and len(rows) == 4 * SHAPES["tiny"].layers * len(passes)
