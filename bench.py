@@ -20,7 +20,7 @@ user calls, with the activations coming from pinned host memory and the results 
 inside the timed region.  `verify` = what the timed launches computed, compared after the timed
 region with a plain fp32 torch dequantise-and-matmul on sampled output columns.  Further legs
 (each a sub-record of the same line; `--legs` selects):
-  overlapped_launches  the headline launches issued alternately on two streams (informational)
+  overlapped_launches  the headline launches issued alternately on two streams, and each waiting for the one in front (informational)
   cta_timeline   (not in the default set; needs the measurement build of the library) per-CTA cycle counters of
                the headline launch: dependency wait, main loop, table builds, waiting for ring data
   small_batch  the same 7B shapes with per-layer bit widths drawn from {2,3,4} (p = 0.3/0.5/0.2)
@@ -367,11 +367,12 @@ class SetRunner:
     """The launches of a LinearSet in one arrangement, on one GPU or column-parallel with the output slices
     gathered either inside the kernel (peer stores + counters) or by NCCL."""
 
-    def __init__(self, lset, per_block_groups, *, peer=None, y_full=None, nslots=4, fixed_acc=False):
+    def __init__(self, lset, per_block_groups, *, peer=None, y_full=None, nslots=4, fixed_acc=False, overlap=True):
         from shiftaddllm_b200 import lutgemm
 
         self.lset, self.peer, self.y_full, self.nslots = lset, peer, y_full, nslots
-        self.overlap = len(per_block_groups) == 1   # several launches per block stand for a chain in which each feeds the next
+        # several launches per block stand for a chain in which each feeds the next
+        self.overlap = overlap and len(per_block_groups) == 1
         self.products = lset.products(per_block_groups)
         if fixed_acc:     # one GPU only: outputs are fixed-point accumulators the products add into (no split-K reduction tail)
             lset.enable_accumulators()
@@ -523,8 +524,11 @@ def run_ours(args, rank, world, device):
         "data": "synthetic", "impl": "ours",
         "config": {"workload": f"{args.workload} decode linear set ({n_layers} blocks x 7 linears), M=1, BCQ {q}-bit g128",
                    "launches_per_step": n_launch,
-                   "launch_structure": ("one grouped launch per decoder block (7 independent products); PDL chained; "
-                                        + ("CUDA graph" if graphed else "eager")),
+                   "launch_structure": ("one grouped launch per decoder block (7 independent products); "
+                                        + ("the blocks read their own activations: each launch computes ahead and waits for the one in "
+                                           "front only before it writes" if head.sequence is not None and head.sequence._overlap else
+                                           "PDL chained, each launch waits for the one in front at its start")
+                                        + "; " + ("CUDA graph" if graphed else "eager")),
                    "l2": f"inputs larger than L2 ({total / 1e9:.1f} GB of weights per step), no flush",
                    "parallelism": (f"column-parallel x{world}, all-gather "
                                    + ("fused into the kernel (peer-to-peer stores + counters)" if fused else "by NCCL"))
@@ -554,6 +558,15 @@ def run_ours(args, rank, world, device):
                              "checker": "fp32 torch dequantise + matmul on the same device tensors"}
             if world > 1:
                 out["exchange_check"] = head.exchange_check()
+
+    # ---- the same launches, each waiting for the one in front at its start (what the headline was before launches computed ahead)
+    if "overlapped_launches" in legs and head.sequence is not None and head.sequence._overlap:
+        chain = SetRunner(lset, HEADLINE_GROUPS, overlap=False)
+        chain_replay, _ = timer.capture(chain.step)
+        chain_ms, _ = timer.timed(chain_replay, args.steps)
+        out["chained_launches"] = {"ms_per_step": round(chain_ms, 4), "value": round(total / (chain_ms * 1e-3) / 1e9, 1), "unit": "GB/s",
+                                   "frac_of_measured_hbm": round(total / (chain_ms * 1e-3) / 1e9 / peak, 4),
+                                   "structure": "the headline launches, PDL chained, each waits for the one in front at its start"}
 
     # ---- the same launches issued alternately on two streams (informational: shows what the wait for the last thread
     # block of the launch in front costs a chain of launches)
@@ -834,7 +847,7 @@ def sharded_decoder_record(args, rank, world, device):
         model = decoder.BcqLlamaDecoder(shape, 2, G, max_len=prompt + 2 * new + 16, device=device, atomic=True)
         r = decoder.benchmark(model, prompt, new)
         rec["batch1_fixed_accumulators"] = {"tokens_per_s": round(r["tokens_per_s"], 1), "ms_per_step": round(r["ms_per_token"], 4),
-                                            "prompt": "prompt fed through the model in chunks of 64 tokens",
+                                            "prompt": "prompt fed through the model in passes of up to 512 tokens",
                                             "structure": "single-GPU decoder, products add into 64-bit fixed-point accumulators"}
         del model
         torch.cuda.empty_cache()
