@@ -80,7 +80,7 @@ class _Block:
 
 def _group(lins, x, outs, pdl=True, x_mul=None, atomic=False, swiglu_fixed=False, many_rows=False):
     """One grouped LUT-GEMV launch: every layer of `lins` applied to the same activation row
-    (`x_mul` given: to silu(x) * x_mul, formed inside the kernel)."""
+    (`x_mul` given: to silu(x) * x_mul, formed in the table build, or for tensor-core rows by a launch in front)."""
     probs = [dict(output=o, bWeight=l.binaryWeight, alpha=l.alpha, bias=l.bias, d_input=x, mSize=l.N, kSize=l.K,
                   nb=l.wbit, num_groups=l.alpha.shape[0], d_input_mul=x_mul) for l, o in zip(lins, outs)]
     lutgemm.lutgemv_grouped(probs, pdl=pdl, atomic_fixed=atomic, swiglu_fixed=swiglu_fixed, many_rows=many_rows)
@@ -431,7 +431,7 @@ class BcqLlamaBatchDecoder:
             _group((blk.o_proj,), self._attn, (self._o,))
             decode_ops.residual_rmsnorm_rows(x, self._o, blk.post_norm, hn, x, s.eps)
             _group((blk.gate_proj, blk.up_proj), hn, (self._gate, self._up))
-            _group((blk.down_proj,), self._gate, (self._down,), x_mul=self._up)   # SiLU(gate)*up formed in the table build
+            _group((blk.down_proj,), self._gate, (self._down,), x_mul=self._up)   # with SiLU(gate)*up as its activation
             delta = self._down
         decode_ops.residual_rmsnorm_rows(x, delta, self.final_norm, hn, x, s.eps)
         self.logits.copy_(torch.matmul(hn, self.lm_head.t()).float())
@@ -460,7 +460,7 @@ class BcqLlamaBatchDecoder:
             x = x + self._o
             hn = F.rms_norm(x, (s.hidden,), blk.post_norm, s.eps)
             _group((blk.gate_proj, blk.up_proj), hn, (self._gate, self._up))
-            _group((blk.down_proj,), self._gate, (self._down,), x_mul=self._up)   # SiLU(gate)*up formed in the table build
+            _group((blk.down_proj,), self._gate, (self._down,), x_mul=self._up)   # with SiLU(gate)*up as its activation
             x = x + self._down
         hn = F.rms_norm(x, (s.hidden,), self.final_norm, s.eps)
         self.logits.copy_(torch.matmul(hn, self.lm_head.t()).float())

@@ -244,8 +244,9 @@ class GroupedLaunch:
 class LaunchSequence:
     """Several prepared launches enqueued by one call into the library (`sal_launch_prepared_sequence`): what a
     decoder block or a whole token is.  All launches must belong to one device.  Where no launch reads what
-    another one of the sequence writes, a launch starts to compute while the one in front of it finishes
-    (`sal_launch_prepared_sequence_overlapped`); ``overlap=False``: each one waits for the one in front at its start."""
+    another one of the sequence writes, a launch starts to compute while the one in front of it finishes, except for the
+    first, which waits for all earlier work of the stream (`sal_launch_prepared_sequence_overlapped`);
+    ``overlap=False``: each one waits for the one in front at its start."""
 
     def __init__(self, launches, overlap: bool = True):
         self._launches = list(launches)
@@ -286,7 +287,7 @@ def lutgemv_grouped(problems, *, pdl=False, accumulate=False, atomic_fixed=False
     """Several independent mode-A products in one launch.  ``problems`` is a list
     of dicts with keys output, bWeight, alpha, bias (or None), d_input,
     mSize, kSize, nb, num_groups and optionally d_input_mul (the activation is then
-    silu(d_input) * d_input_mul, computed while the tables are built).
+    silu(d_input) * d_input_mul, formed while the tables are built or, for tensor-core rows, by a launch in front).
 
     ``atomic_fixed=True``: every ``output`` is an int64 fixed-point accumulator (units of 2**-32, see
     :data:`FIXED_ONE`) the product is ADDED to with integer atomics: no split-K reduction tail, and — integer
