@@ -26,9 +26,9 @@
 //   warp 21     issues tcgen05.mma (M = 128 output columns, N = rows, K = 16) and commits
 //   warp 22     activations by tiled TMA into 128-byte-swizzled shared memory (operand B)
 //
-// Work split: the launch's (output tile, 128-feature unit) pairs in tile-major order are dealt to the CTAs in equal
-// contiguous runs.  A tile that several CTAs share is summed by the last of them to arrive, in ascending order of K
-// (deterministic), from fp32 partial sums in the scratch buffer.
+// Work split: the launch's (output tile, 128-feature unit) pairs in tile-major order are dealt to the CTAs in contiguous runs: whole
+// numbers of CTAs per tile where that fills most of the SMs (whole_shares), else equal runs that may end inside a tile.  A tile that several CTAs
+// share is summed by the last of them to arrive, in ascending order of K (deterministic), from fp32 partial sums in the scratch buffer.
 //
 // What bounds it: a unit takes 0.66 / 0.9 / 1.1 us for 2 / 3 / 4 planes up to 64 rows, against 0.13 to 0.26 us that its planes take to
 // arrive.  About half of that the MMA warp waits for activations and the operand warps for the stages it frees; the operands
