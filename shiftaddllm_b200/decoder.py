@@ -177,7 +177,7 @@ class BcqLlamaDecoder:
     def _step_fused(self):
         """Same step with the fused helpers of include/sal_decode_ops.h: per block 4 LUT-GEMV
         launches + 4 helper launches (residual+RMSNorm x2, RoPE+cache write, attention); SiLU(gate)*up is
-        computed inside down_proj's table build."""
+        formed in down_proj's table build."""
         s = self.shape
         hd, kvh = s.head_dim, s.kv_heads
         scale = 1.0 / math.sqrt(hd)
@@ -332,7 +332,8 @@ class BcqLlamaDecoder:
                 _group((blk.gate_proj, blk.up_proj), hn, (gate, up), many_rows=many)
                 _group((blk.down_proj,), gate, (down,), x_mul=up, many_rows=many)   # with SiLU(gate)*up as its activation
                 delta = down
-            x = x + down
+            if delta is not None:
+                x = x + delta
         hn = F.rms_norm(x[-1:], (h,), self.final_norm, s.eps)
         self.logits.copy_(torch.matmul(hn, self.lm_head.t()).float().view(-1))
         self.token.copy_(self.logits.argmax().view(1))

@@ -7,7 +7,7 @@ import pytest
 import torch
 
 from shiftaddllm_b200 import decode_ops
-from shiftaddllm_b200.decoder import SHAPES, BcqLlamaDecoder
+from shiftaddllm_b200.decoder import SHAPES, BcqLlamaDecoder, LlamaShape
 
 pytestmark = pytest.mark.gpu
 
@@ -79,3 +79,13 @@ def test_chunk_is_the_bound_on_the_rows_of_a_pass(chunk, passes, monkeypatch):
     model = BcqLlamaDecoder(SHAPES["tiny"], 3, 128, max_len=160)
     model.feed(list(range(150)), **({} if chunk is None else {"chunk": chunk}))
     assert rows[::4 * SHAPES["tiny"].layers] == passes and len(rows) == 4 * SHAPES["tiny"].layers * len(passes)
+
+
+def test_prompt_through_a_model_without_blocks():
+    """Embedding, final norm and head alone: nothing is added that no block has written."""
+    shape = LlamaShape(256, 0, 2, 2, 512, vocab=1000)
+    model = BcqLlamaDecoder(shape, 3, 128, max_len=16)
+    torch.full((1 << 20,), float("nan"), dtype=torch.float16, device="cuda")   # what freed memory then holds
+    model.feed([1, 2, 3])
+    want = torch.nn.functional.rms_norm(model.embed[3], (256,), model.final_norm, shape.eps) @ model.lm_head.t()
+    assert (model.logits - want.float()).norm() <= 2.0 ** -9 * want.float().norm()
